@@ -57,12 +57,16 @@ enum : int { TOPO_FATTREE = 0, TOPO_LEAFSPINE = 1, TOPO_GRAPH = 2 };
 #endif
 constexpr int RUNS = TB_CHAIN_RUNS;
 
-struct Chain
+// A run is one 32-bit word (code in the low half, repetitions in the high one), so that a chain is
+// copied, shifted and compared by whole words: a chain is made per frame started and per frame
+// received, and moving its codes and counts as separate 16-bit fields was most of an event's
+// instructions and memory accesses.
+struct alignas(8) Chain
 {
-    uint16_t code[RUNS];
-    uint16_t cnt[RUNS];
-    uint16_t rhi, rlo; // root key (0: none)
+    uint32_t run[RUNS]; // newest first (0: none)
+    uint32_t root;      // root key (0: none)
 };
+static_assert(sizeof(Chain) == 4 * (RUNS + 1), "a chain is whole 8-byte words");
 
 constexpr uint16_t CODE_NOW = 1, CODE_STEP = 2;
 TB_HD uint16_t code_tc(int len) { return (uint16_t)len; }
@@ -76,80 +80,71 @@ TB_HD uint16_t code_lead(int64_t lead_ps)
 TB_HD void chain_clear(Chain &c)
 {
     for (int i = 0; i < RUNS; i++)
-        c.code[i] = 0, c.cnt[i] = 0;
-    c.rhi = c.rlo = 0;
+        c.run[i] = 0;
+    c.root = 0;
 }
 // an application start: host by host, then by connection (world-local ids)
 TB_HD void chain_app_root(Chain &c, int host, int conn)
 {
     chain_clear(c);
-    c.rhi = (uint16_t)(0x8000 | (host + 1));
-    c.rlo = (uint16_t)conn;
+    c.root = (uint32_t)(0x8000 | (host + 1)) << 16 | (uint16_t)conn;
 }
 // a message write (FlowSender::SendMessage), scheduled in main() before the starts
 TB_HD void chain_msg_root(Chain &c, int msg)
 {
     chain_clear(c);
-    c.rhi = (uint16_t)(1 + (msg >> 16));
-    c.rlo = (uint16_t)msg;
+    c.root = (uint32_t)(1 + (msg >> 16)) << 16 | (uint16_t)msg;
 }
 // dst = the chain of an event that `parent` schedules with the lead `code`; dst may be parent
+// (no branch: the parent's words are read once, and each word of dst is one of two of them)
 TB_HD void chain_child(Chain &dst, const Chain &parent, uint16_t code)
 {
-    if (parent.code[0] == code)
-    {
-        if (&dst != &parent)
-            dst = parent;
-        if (dst.cnt[0] < 0xFFFF)
-            dst.cnt[0]++;
-        return;
-    }
-    for (int i = RUNS - 1; i >= 1; i--)
-    {
-        dst.code[i] = parent.code[i - 1];
-        dst.cnt[i] = parent.cnt[i - 1];
-    }
-    dst.code[0] = code;
-    dst.cnt[0] = 1;
-    dst.rhi = parent.rhi;
-    dst.rlo = parent.rlo;
+    const Chain p = parent;
+    const bool same = (p.run[0] & 0xFFFFu) == code;
+    const uint32_t more = p.run[0] < 0xFFFF0000u ? p.run[0] + 0x10000u : p.run[0]; // (the count saturates)
+    Chain d;
+    d.run[0] = same ? more : 0x10000u | code;
+#pragma unroll
+    for (int i = 1; i < RUNS; i++)
+        d.run[i] = same ? p.run[i] : p.run[i - 1];
+    d.root = p.root;
+    dst = d;
 }
 // < 0: a runs first, > 0: b runs first, 0: the recorded histories do not tell
 TB_HDI int chain_cmp(const Chain &a, const Chain &b)
 {
     int ia = 0, ib = 0;
-    uint32_t ra = a.cnt[0], rb = b.cnt[0];
+    uint32_t wa = a.run[0], wb = b.run[0]; // the runs compared, their high halves the repetitions left
     for (;;)
     {
-        uint16_t ca = a.code[ia], cb = b.code[ib];
-        if (ca == 0 && cb != 0 && a.rhi != 0)
+        const uint32_t ca = wa & 0xFFFFu, cb = wb & 0xFFFFu;
+        if (ca == 0 && cb != 0 && a.root >> 16 != 0)
             return -1; // a reached its root, which precedes any other parent
-        if (cb == 0 && ca != 0 && b.rhi != 0)
+        if (cb == 0 && ca != 0 && b.root >> 16 != 0)
             return 1;
         if (ca == 0 || cb == 0)
             break;
         if (ca != cb)
             return ca > cb ? -1 : 1; // the larger lead: the earlier parent
-        uint32_t m = ra < rb ? ra : rb;
-        ra -= m;
-        rb -= m;
-        if (ra == 0)
+        const uint32_t na = wa >> 16, nb = wb >> 16, m = na < nb ? na : nb;
+        wa -= m << 16;
+        wb -= m << 16;
+        if (na == m)
         {
             if (++ia == RUNS)
                 break;
-            ra = a.cnt[ia];
+            wa = a.run[ia];
         }
-        if (rb == 0)
+        if (nb == m)
         {
             if (++ib == RUNS)
                 break;
-            rb = b.cnt[ib];
+            wb = b.run[ib];
         }
     }
-    uint32_t xa = (uint32_t)a.rhi << 16 | a.rlo, xb = (uint32_t)b.rhi << 16 | b.rlo;
-    if (xa == 0 || xb == 0 || xa == xb)
+    if (a.root == 0 || b.root == 0 || a.root == b.root)
         return 0;
-    return xa < xb ? -1 : 1;
+    return a.root < b.root ? -1 : 1;
 }
 
 // ------------------------------------------------------------------ the frame
