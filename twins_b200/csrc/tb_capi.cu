@@ -788,20 +788,20 @@ int make_world(const tb_topology *topo, int n_flows, const int *src, const int *
 }
 
 // the grid of a launch shape: a warp per unit, at most what is co-resident (0: does not fit)
-int grid_for(const tb_ctx *c, int host_lanes, int stage, int units = -1, bool port_local = false, bool free = false)
+int grid_for(const tb_ctx *c, int host_lanes, int stage, int units = -1, bool free = false)
 {
     if (units < 0)
         units = (c->sim.H + host_lanes - 1) / host_lanes + c->sim.S;
-    return grid_of(units, TB_WARPS_PER_BLOCK, tb::slot_kernel_blocks_per_sm(stage, port_local, host_lanes, free), c->dev_sms, c->grid_req);
+    return grid_of(units, TB_WARPS_PER_BLOCK, tb::slot_kernel_blocks_per_sm(stage, host_lanes, free), c->dev_sms, c->grid_req);
 }
 
 // the launch-shape tuner's start, on this context's device: the candidates that fit, and the warps
 // co-resident at one host per warp and the default staging
 void tuner_init(ShapeTuner &tu, const tb_ctx *c, bool autotune, int lanes, int stage, long long entities, int kmax = 0)
 {
-    const long long resident = (long long)c->dev_sms * std::max(1, tb::slot_kernel_blocks_per_sm(SW_STAGE, false, 1)) * TB_WARPS_PER_BLOCK;
+    const long long resident = (long long)c->dev_sms * std::max(1, tb::slot_kernel_blocks_per_sm(SW_STAGE, 1)) * TB_WARPS_PER_BLOCK;
     tu.init(autotune, lanes, stage, c->port_local, entities, kmax, resident,
-            [c](int l, int st, bool pl) { return grid_for(c, l, st, -1, pl) > 0; });
+            [c](int l, int st, bool) { return grid_for(c, l, st) > 0; });
 }
 
 int prepare(tb_ctx *c)
@@ -1163,8 +1163,6 @@ int tb_set_port_local(tb_ctx *ctx, int on)
     if (!ctx)
         return fail(TB_ERR_ARG, "ctx is NULL");
     ctx->port_local = on != 0;
-    if (ctx->prepared && !ctx->autotune && (ctx->grid = grid_for(ctx, ctx->host_lanes, ctx->stage_cap, -1, ctx->port_local)) <= 0)
-        return fail(TB_ERR_CUDA, "the slot kernel does not fit on the device with this shape");
     return TB_OK;
 }
 
@@ -1246,7 +1244,7 @@ int tb_run(tb_ctx *ctx, long long max_slots)
             if (explore ? !tu.probes(k) : k != tu.best)
                 continue;
             ShapeTuner::Shape &sh = tu.shapes[k];
-            int grid = ctx->grid_req > 0 && !ctx->autotune ? ctx->grid : grid_for(ctx, sh.lanes, sh.stage, -1, sh.port_local);
+            int grid = ctx->grid_req > 0 && !ctx->autotune ? ctx->grid : grid_for(ctx, sh.lanes, sh.stage);
             if (free)
             {
                 if (alive != list_alive || sh.lanes != list_lanes)
@@ -1261,7 +1259,7 @@ int tb_run(tb_ctx *ctx, long long max_slots)
                 }
                 s.unit_list = ctx->d_units;
                 s.n_list = (int)ulist.size();
-                grid = grid_for(ctx, sh.lanes, sh.stage, s.n_list, sh.port_local, true);
+                grid = grid_for(ctx, sh.lanes, sh.stage, s.n_list, true);
                 if (ctx->grid_req > 0 && !ctx->autotune)
                     grid = std::min(grid, ctx->grid);
             }
@@ -1278,14 +1276,14 @@ int tb_run(tb_ctx *ctx, long long max_slots)
                 }
                 s.unit_list = ctx->d_units;
                 s.n_list = (int)ulist.size();
-                grid = grid_for(ctx, sh.lanes, sh.stage, s.n_list, sh.port_local);
+                grid = grid_for(ctx, sh.lanes, sh.stage, s.n_list);
             }
             const long long slots_before = ctl.slots_run;
             cudaEventRecord(ctx->la, ctx->stream);
             // (the steady launches replay a captured graph; the short probes launch directly)
-            int e = explore ? (free ? tb::launch_free(s, grid, tu.probe, sh.lanes, sh.stage, sh.port_local, ctx->stream)
-                                    : tb::launch_slots(s, grid, tu.probe, sh.lanes, sh.stage, sh.port_local, ctx->stream))
-                            : tb::launch_slots_graph(graph, s, grid, run_slots, sh.lanes, sh.stage, sh.port_local, ctx->stream, free);
+            int e = explore ? (free ? tb::launch_free(s, grid, tu.probe, sh.lanes, sh.stage, ctx->stream)
+                                    : tb::launch_slots(s, grid, tu.probe, sh.lanes, sh.stage, ctx->stream))
+                            : tb::launch_slots_graph(graph, s, grid, run_slots, sh.lanes, sh.stage, ctx->stream, free);
             if (e)
                 return fail(TB_ERR_CUDA, std::string("slot kernel launch: ") + cudaGetErrorString((cudaError_t)e));
             cudaEventRecord(ctx->lb, ctx->stream);
@@ -1328,7 +1326,7 @@ int tb_run(tb_ctx *ctx, long long max_slots)
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     ctx->ran = true;
     const ShapeTuner::Shape &most = tu.shapes[tu.most()];
-    const int most_grid = grid_for(ctx, most.lanes, most.stage, -1, most.port_local);
+    const int most_grid = grid_for(ctx, most.lanes, most.stage);
 #ifdef TB_PROFILE
     if (ctl.slots_run > 1)
     {
@@ -1581,7 +1579,7 @@ extern "C" int tb_run_static(int device, const tb_topology *topo, int n_flows, c
     SlotCtl ctl{};
     for (;;)
     {
-        int e = tb::launch_slots(s, c.grid, c.max_slots_per_launch, c.host_lanes, c.stage_cap, false, 0);
+        int e = tb::launch_slots(s, c.grid, c.max_slots_per_launch, c.host_lanes, c.stage_cap, 0);
         if (e)
             return fail(TB_ERR_CUDA, std::string("slot kernel launch: ") + cudaGetErrorString((cudaError_t)e));
         if (cudaMemcpy(&ctl, s.ctl, sizeof ctl, cudaMemcpyDeviceToHost) != cudaSuccess)

@@ -92,16 +92,40 @@ TB_D int msg_count(const Sim &s, int64_t slot, int link)
 }
 TB_D const Frame *msg_frames(const Sim &s, int64_t slot, int link) { return s.msg + msg_index(s, slot, link) * MAX_TX; }
 
+#ifdef TB_QTRACE
+// the enqueue trace: frame g joined the queue disc of (node, dev) at `now` behind `backlog` frames
+TB_D void qtrace_enqueue(const Sim &s, int node, int dev, const Frame &g, int backlog, int64_t now)
+{
+    if (!s.qtrace || now >= s.qtrace_until || now < s.qtrace_from)
+        return;
+#if defined(__CUDA_ARCH__)
+    const unsigned long long i = atomicAdd(s.qtrace_cnt, 1ull);
+#else
+    const unsigned long long i = (*s.qtrace_cnt)++;
+#endif
+    if (i >= s.qtrace_n)
+        return;
+    QRec &r = s.qtrace[i];
+    const SndRec &S = s.snd[g.flow];
+    r.ts = now;
+    r.node = node;
+    r.dev = dev;
+    r.src = g.to_sender ? S.dst_local : S.src_local;
+    r.dst = g.to_sender ? S.src_local : S.dst_local;
+    r.sa = g.sa;
+    r.len = g.len;
+    r.qlen = (uint16_t)(backlog + 1);
+    r.flags = g.flags;
+}
+#endif
+
 // The sending end of a point-to-point link for one slot: ns-3's RED queue disc over a one-packet
 // device queue over the wire (reference: src/step.cuh:163-317). `ring` holds the frames that have
 // not started, each stamped with its enqueue time; the wire is busy until `busy_until` with the
 // frame that began at `began`, whose chain is *tx_chain. A frame begins at max(its enqueue time,
 // busy_until); its transmission's copy, stamped with its arrival at the far end, goes to this
 // slot's link message `msg` (at most MAX_TX; more is counted as an overflow).
-// SHADOW: the frame enqueued last is also kept at *shadow (shared memory) with its ring index, so
-// that a frame queued and started in the same slot is not read back from global memory.
-template <bool SHADOW>
-struct Transmitter
+struct Egress
 {
     Frame *ring;
     int cap, head, size;
@@ -114,8 +138,6 @@ struct Transmitter
     Frame *msg;
     int n_out;
     unsigned drops, marks, ovf, offered;
-    Frame *shadow;
-    int shadow_at;
 #ifdef TB_QTRACE
     const Sim *qs; // the trace's sink; the queue's ns-3 node and device
     int qnode, qdev;
@@ -138,10 +160,7 @@ struct Transmitter
         msg = msg_;
         n_out = 0;
         drops = marks = ovf = offered = 0;
-        shadow = nullptr;
-        shadow_at = -1;
     }
-    TB_D const Frame &at_head() const { return SHADOW && head == shadow_at ? *shadow : ring[head]; }
 
     // every waiting frame that begins by `until` (and before the horizon) goes on the wire; a frame
     // that found the wire busy begins at the previous one's TransmitComplete, whose chain is its
@@ -150,7 +169,7 @@ struct Transmitter
     {
         for (; size; size--)
         {
-            const Frame &f = at_head();
+            const Frame &f = ring[head];
             const int64_t t0 = f.ts > busy_until ? f.ts : busy_until;
             if (t0 > until || t0 >= horizon)
                 return;
@@ -189,32 +208,6 @@ struct Transmitter
         return size - (woken ? 1 : 0);
     }
 
-#ifdef TB_QTRACE
-    TB_D void trace(const Frame &g, int backlog, int64_t now) const
-    {
-        if (!qs->qtrace || now >= qs->qtrace_until || now < qs->qtrace_from)
-            return;
-#if defined(__CUDA_ARCH__)
-        const unsigned long long i = atomicAdd(qs->qtrace_cnt, 1ull);
-#else
-        const unsigned long long i = (*qs->qtrace_cnt)++;
-#endif
-        if (i >= qs->qtrace_n)
-            return;
-        QRec &r = qs->qtrace[i];
-        const SndRec &S = qs->snd[g.flow];
-        r.ts = now;
-        r.node = qnode;
-        r.dev = qdev;
-        r.src = g.to_sender ? S.dst_local : S.src_local;
-        r.dst = g.to_sender ? S.src_local : S.dst_local;
-        r.sa = g.sa;
-        r.len = g.len;
-        r.qlen = (uint16_t)(backlog + 1);
-        r.flags = g.flags;
-    }
-#endif
-
     // a frame offered at `now` (its ts becomes now): the wire first takes what begins by now; RED
     // with MinTh = MaxTh = K and weight 1 (no averaging) marks an ECT frame or drops another when
     // the backlog is at least K (and above 1); then the disc's limit drops. False: dropped.
@@ -240,7 +233,7 @@ struct Transmitter
             return false;
         }
 #ifdef TB_QTRACE
-        trace(g, backlog, now);
+        qtrace_enqueue(*qs, qnode, qdev, g, backlog, now);
 #endif
         if (size == cap)
         {
@@ -249,16 +242,8 @@ struct Transmitter
         }
         const int at = head + size < cap ? head + size : head + size - cap;
         frame_copy(&ring[at], &g);
-        if (SHADOW)
-        {
-            *shadow = g;
-            shadow_at = at;
-        }
         size++;
         return true;
     }
 };
-using Egress = Transmitter<false>;
-using PortEgress = Transmitter<true>;
-
 } // namespace tb

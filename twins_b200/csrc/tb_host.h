@@ -98,7 +98,7 @@ struct ShapeTuner
         int lanes, stage;
         long long slots;
         int strikes;
-        bool port_local; // switch ports' slot copies in shared memory (PortEgress)
+        bool port_local; // (every shape keeps a port's slot state on chip: a label of the shape)
     };
     std::vector<Shape> shapes;
     size_t best = 0;
@@ -128,8 +128,8 @@ struct ShapeTuner
             for (auto &x : CAND)
                 if (fits(x[0], x[1], x[2] != 0))
                     shapes.push_back({x[0], x[1], 0, 0, x[2] != 0});
-            // (one host per warp: with big switches (16 ports or more), whose ports' serial
-            // enqueues are the critical path, the port-local egress and the largest staging; else
+            // (one host per warp: with big switches (16 ports or more), whose ports'
+            // enqueues are the critical path, the largest staging (and its label); else
             // the largest staging that keeps two blocks per SM. 32 hosts per warp: the smallest
             // staging, for four blocks per SM)
             const int lanes0 = entities <= 2 * resident ? 1 : 32;

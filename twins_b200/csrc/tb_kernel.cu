@@ -50,214 +50,6 @@ __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefe
 // the stream's look-ahead rows (tb_common.cuh), in global memory, read through the read-only path
 __device__ const RngAhead g_rng_ahead = make_rng_ahead();
 
-// Per-packet spraying's draws with staged frames: the merged arrival order, then the draws. Each
-// frame's (time, longer first) is one 32-bit key (its offset in the slot, 21 bits; 2047 - its
-// length, 11 bits), so a merge step is one warp-wide minimum of the ports' head keys; frames that tie
-// on the key are ordered by lane 0 exactly as the serial merge (sw_phase_spray) orders them, scanning
-// the tied ports in port order. The merge only records the order: a prefix over it gives each
-// drawing frame its place among the slot's draws, and every draw is then computed at once, from the
-// stream's state and the look-ahead rows. Returns false, having written nothing but the warp's
-// scratch, when a frame's key does not fit (the argmin merge below then runs). The scratch: the
-// windows' flat starts in base (phase 5 writes it afterwards); keys, then places, in the egress
-// sources region; the merge order and each frame's draw kind in the egress times region.
-__device__ bool sw_spray_keyed(const SwCtx &x, SwShared &sh, int lane, unsigned &ties)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int k = x.sr->k;
-    const WorldDesc &wd = *x.wd;
-    const int64_t S0 = x.t * SLOT_PS;
-    const Input in = input_of(x, sh, lane < k ? lane : 0);
-    const int c = lane < k ? in.count() : 0;
-    int incl = c;
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        const int v = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o)
-            incl += v;
-    }
-    const int total = __shfl_sync(FULL, incl, 31), base = incl - c;
-    if (total == 0)
-        return true;
-    if (total > RNG_AHEAD)
-        return false;
-    uint32_t *key = sh.eref();                            // [total]: keys, then places
-    int *ord = reinterpret_cast<int *>(sh.ets());         // [total]: flat frames in merge order
-    int *kind = reinterpret_cast<int *>(sh.ets()) + sh.cap; // [total]: 0 port down, 1 no routes (0 written), nr + 1
-    if (lane < k)
-        sh.base[lane] = base;
-    bool bad = false;
-    for (int j = 0; j < c; j++)
-    {
-        const Frame &f = *in.at(j);
-        const int64_t off = f.ts - S0;
-        bad |= off < 0 || off >= (1 << 21) || f.len > 2047;
-        key[base + j] = (uint32_t)off << 11 | (uint32_t)(2047 - f.len);
-        const int ep = wd.n_fail ? epoch_of(wd, f.ts) : 0;
-        kind[base + j] = port_down(wd, x.sr->local, lane, ep) ? 0 : 1 + routes_to(wd, x.sr->local, f.dst, ep);
-    }
-    if (__any_sync(FULL, bad))
-        return false;
-    __syncwarp();
-    int pos = 0;
-    uint32_t head = c ? key[base] : 0xFFFFFFFFu;
-    for (int r = 0; r < total; r++)
-    {
-        const uint32_t m = __reduce_min_sync(FULL, head);
-        const unsigned cand = __ballot_sync(FULL, head == m);
-        int best = __ffs(cand) - 1;
-        if (cand & (cand - 1))
-        {
-            // equal times and lengths: the upstream chains, then the connection id
-            const Frame *bf = nullptr;
-            for (unsigned cc = cand; cc; cc &= cc - 1)
-            {
-                const int q = __ffs(cc) - 1;
-                const int pq = __shfl_sync(FULL, pos, q);
-                if (lane == 0)
-                {
-                    const Frame *f = input_of(x, sh, q).at(pq);
-                    if (!bf || frame_before(*f, *bf, ties))
-                    {
-                        best = q;
-                        bf = f;
-                    }
-                }
-            }
-            best = __shfl_sync(FULL, best, 0);
-        }
-        if (lane == best)
-        {
-            ord[r] = base + pos;
-            pos++;
-            head = pos < c ? key[base + pos] : 0xFFFFFFFFu;
-        }
-    }
-    __syncwarp();
-    // places among the draws: an exclusive prefix of the drawing frames in merge order
-    int run = 0;
-    for (int r0 = 0; r0 < total; r0 += 32)
-    {
-        const int r = r0 + lane, i = r < total ? ord[r] : 0, v = r < total && kind[i] >= 2;
-        int sc = v;
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int u = __shfl_up_sync(FULL, sc, o);
-            if (lane >= o)
-                sc += u;
-        }
-        if (r < total)
-            key[i] = run + sc - v;
-        run += __shfl_sync(FULL, sc, 31);
-    }
-    __syncwarp();
-    const Rng st = x.s->sw_rng[x.sw];
-    for (int i = lane; i < total; i += 32)
-    {
-        const int v = kind[i];
-        if (v == 0)
-            continue;
-        int q = 0;
-        while (q + 1 < k && sh.base[q + 1] <= i)
-            q++;
-        uint8_t u = 0;
-        if (v >= 2)
-        {
-            const uint32_t *row = g_rng_ahead.r[key[i] + 1];
-            u = (uint8_t)int_of_u01(u01_of(rng_ahead_value<RNG_M1>(row, st.s), rng_ahead_value<RNG_M2>(row + 3, st.s + 3)), (uint32_t)(v - 1));
-        }
-        x.s->sw_up[x.scratch + (size_t)q * 2 * MAX_TX + (i - sh.base[q])] = u;
-    }
-    // the stream after the slot's draws: each component's last three values
-    __syncwarp(); // (every lane has read the stream)
-    if (lane < 6)
-    {
-        const int cmp = lane / 3, m = run - 2 + lane % 3;
-        const uint32_t *row = g_rng_ahead.r[m > 0 ? m : 1] + 3 * cmp;
-        x.s->sw_rng[x.sw].s[lane] = m <= 0 ? st.s[3 * cmp + m + 2]
-                                           : (cmp ? rng_ahead_value<RNG_M2>(row, st.s + 3) : rng_ahead_value<RNG_M1>(row, st.s));
-    }
-    return true;
-}
-
-// Per-packet spraying's draws with staged frames whose keys do not fit (sw_spray_keyed): the merged
-// arrival order by a warp-wide argmin of (time, length), one draw after another.
-// Lane q holds port q's next frame; the minimum (time, longer first) wins; frames that tie on
-// both are ordered by lane 0 exactly as the serial merge (sw_phase_spray) orders them, scanning
-// the tied ports in port order. Lane 0 keeps the switch's random stream and draws.
-__device__ void sw_phase_spray_warp(const SwCtx &x, const SwShared &sh, int lane, unsigned &ties)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int k = x.sr->k;
-    const WorldDesc &wd = *x.wd;
-    Input in{};
-    int cnt = 0, pos = 0;
-    if (lane < k)
-    {
-        in = input_of(x, sh, lane);
-        cnt = in.count();
-    }
-    Rng st;
-    if (lane == 0)
-        st = x.s->sw_rng[x.sw];
-    for (;;)
-    {
-        const bool has = lane < k && pos < cnt;
-        long long kts = has ? in.at(pos)->ts : LLONG_MAX;
-        int klen = has ? in.at(pos)->len : 0;
-        long long mts = kts;
-        int mlen = klen;
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            long long ots = __shfl_xor_sync(FULL, mts, o);
-            int olen = __shfl_xor_sync(FULL, mlen, o);
-            if (ots < mts || (ots == mts && olen > mlen))
-            {
-                mts = ots;
-                mlen = olen;
-            }
-        }
-        if (mts == LLONG_MAX)
-            break;
-        const unsigned cand = __ballot_sync(FULL, has && kts == mts && klen == mlen);
-        int best = __ffs(cand) - 1;
-        if (cand & (cand - 1))
-        {
-            // equal times and lengths: the upstream chains, then the connection id
-            const Frame *bf = nullptr;
-            for (unsigned c = cand; c; c &= c - 1)
-            {
-                int q = __ffs(c) - 1;
-                int pq = __shfl_sync(FULL, pos, q);
-                if (lane == 0)
-                {
-                    const Frame *f = input_of(x, sh, q).at(pq);
-                    if (!bf || frame_before(*f, *bf, ties))
-                    {
-                        best = q;
-                        bf = f;
-                    }
-                }
-            }
-            best = __shfl_sync(FULL, best, 0);
-        }
-        const int pb = __shfl_sync(FULL, pos, best);
-        if (lane == 0)
-        {
-            const Frame &w = *input_of(x, sh, best).at(pb);
-            int ep = wd.n_fail ? epoch_of(wd, w.ts) : 0;
-            if (!port_down(wd, x.sr->local, best, ep))
-            {
-                int nr = routes_to(wd, x.sr->local, w.dst, ep);
-                x.s->sw_up[x.scratch + (size_t)best * 2 * MAX_TX + pb] = (uint8_t)(nr ? rand_int(st, (uint32_t)nr) : 0);
-            }
-        }
-        if (lane == best)
-            pos++;
-    }
-    if (lane == 0)
-        x.s->sw_rng[x.sw] = st;
-}
-
 // The world's rule for this slot (reference src/kernel.cuh:79-112, per world): the next launch
 // slot its entities run, and its time origin; both read through L2 (the controller of another SM
 // writes them)
@@ -497,9 +289,9 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
                 at -= s.ring;
             prefetch_l1(&s.host_ring[(size_t)h * s.ring + at]);
         }
-        if (sh.cap * (int)(sizeof(int64_t) + sizeof(uint32_t)) >= DUE_CAP * (int)sizeof(Due))
+        if (sh.due_fit(DUE_CAP * sizeof(Due)))
         {
-            due = reinterpret_cast<Due *>(sh.ets()); // (the egress regions, unused by a host)
+            due = reinterpret_cast<Due *>(sh.due_area()); // (the word arrays, unused by a host)
             due_n = collect_due_warp(s, hr, h, (t - t0 + 1) * SLOT_PS, lane, due, &due_ovf);
         }
         else
@@ -571,73 +363,21 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
     __syncwarp(); // (the staging area is reused by the warp's next unit)
 }
 
-// one switch, one slot (launch slot gt), by its warp (lanes >= k idle but take part in the warp
-// barriers); nothing when its world does not run this slot
-template <bool PORT_LOCAL>
-__device__ bool switch_step(const Sim &s, int sw, int64_t gt, int lane, SwShared &sh, unsigned &ties)
+// a slot's messages beyond the staging area: the phases through L2, a port per lane
+__device__ __noinline__ bool switch_unstaged(const SwCtx &x, SwShared &sh, int lane, SwCounts &c)
 {
-    const SwRec &sr = s.sws[sw];
-    const int64_t next = world_next(s, sr.world), t0 = world_t0(s, sr.world);
-    const int64_t t = gt - t0;
-    SwCtx x;
-    x.s = &s;
-    x.wd = &s.worlds[sr.world];
-    x.sr = &sr;
-    x.sw = sw;
-    x.ports = s.ports + sr.port0;
-    x.scratch = (size_t)sw * s.kmax * 2 * MAX_TX;
-    x.t = t;
-    x.gt = gt;
-    x.spray = x.wd->spray != 0;
-    const int k = sr.k;
-    const bool on = lane < k;
-    unsigned pk = 0, drops = 0, marks = 0, ovf = 0, my_ties = 0;
-#ifdef TB_PROFILE
-    unsigned long long sp0 = globaltimer();
-#endif
+    const bool on = lane < x.sr->k;
     if (on)
-        sw_phase_sizes(x, sh, lane);
-    // its world does not run this slot; or no frame arriving and every queue empty: nothing to do
-    // (its link messages of this slot stay unwritten, and a stale tag reads as an empty message)
-    if (gt < next || !__any_sync(0xffffffffu, on && (sh.raw2[lane] | sh.raw1[lane] | x.ports[lane].q_size) != 0))
-        return false;
+        c.pk = sw_phase_window(x, sh, lane);
     __syncwarp();
-    if (lane == 0)
-        sw_phase_layout(x, sh);
-    __syncwarp();
-    sw_phase_copy(x, sh, lane, 32);
-    __syncwarp();
-    if (on)
-        pk = sw_phase_window(x, sh, lane);
-    __syncwarp();
-#ifdef TB_PROFILE
-    unsigned long long sp2 = globaltimer();
-    if (lane == 0)
-        atomicAdd(&s.ctl->prof_phase[11], sp2 - sp0);
-#endif
     if (x.spray)
     {
-        if (sh.staged)
-        {
-            const bool keyed = sw_spray_keyed(x, sh, lane, my_ties);
-#ifdef TB_PROFILE
-            if (lane == 0)
-                atomicAdd(&s.ctl->prof_phase[keyed ? 13 : 14], 1000ull);
-#endif
-            if (!keyed)
-                sw_phase_spray_warp(x, sh, lane, my_ties);
-        }
-        else if (lane == 0)
-            sw_phase_spray(x, sh, my_ties);
+        if (lane == 0)
+            sw_phase_spray(x, sh, c.ties);
         __syncwarp();
     }
-#ifdef TB_PROFILE
-    unsigned long long sp3 = globaltimer();
-    if (lane == 0)
-        atomicAdd(&s.ctl->prof_phase[12], sp3 - sp2);
-#endif
     if (on)
-        drops += sw_phase_count(x, sh, lane);
+        c.drops += sw_phase_count(x, sh, lane);
     __syncwarp();
     if (on)
         sw_phase_offsets(x, sh, lane);
@@ -648,44 +388,213 @@ __device__ bool switch_step(const Sim &s, int sw, int64_t gt, int lane, SwShared
     if (on)
         sw_phase_scatter(x, sh, lane);
     __syncwarp();
-#ifdef TB_PROFILE
-    unsigned long long sp1 = globaltimer();
-    if (lane == 0)
-        atomicAdd(&s.ctl->prof_phase[6], sp1 - sp0);
-#endif
-    bool act = false;
-    if (on)
-        act = sw_phase_egress<PORT_LOCAL>(x, sh, lane, my_ties, drops, marks, ovf);
-    __syncwarp();
-#ifdef TB_PROFILE
-    if (lane == 0)
-        atomicAdd(&s.ctl->prof_phase[7], globaltimer() - sp1);
-#endif
-    // warp totals, one atomic each
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        pk += __shfl_xor_sync(0xffffffffu, pk, o);
-        drops += __shfl_xor_sync(0xffffffffu, drops, o);
-        marks += __shfl_xor_sync(0xffffffffu, marks, o);
-        ovf += __shfl_xor_sync(0xffffffffu, ovf, o);
-        my_ties += __shfl_xor_sync(0xffffffffu, my_ties, o);
-    }
-    bool any = __any_sync(0xffffffffu, act);
-    if (lane == 0)
-    {
-        ev_add(s, sr.world, EV_SW_PKT, pk);
-        ev_add(s, sr.world, EV_DROPS, drops);
-        ev_add(s, sr.world, EV_MARKS, marks);
-        ev_add(s, sr.world, EV_OVF_TX, ovf);
-        ev_add(s, sr.world, EV_TIES, my_ties);
-        ties += my_ties;
-    }
-    return any;
+    return on && sw_phase_egress(x, sh, lane, c);
 }
 
-// PORT_LOCAL: switch ports keep the slot's transmission chain and last enqueued frame in shared
-// memory (PortEgress); MIN_BLOCKS: the register budget. Separate instantiations, chosen per launch.
-template <bool PORT_LOCAL, int MIN_BLOCKS>
+// one switch, one slot (launch slot gt), by its warp; nothing when its world does not run this slot
+__device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, int lane, SwShared &sh, unsigned &ties)
+{
+    const unsigned FULL = 0xffffffffu;
+    const SwRec &sr = s.sws[sw];
+    const int64_t next = world_next(s, sr.world), t0 = world_t0(s, sr.world);
+    const int k = sr.k;
+    const bool on = lane < k;
+    int link = -1, n2 = 0, n1 = 0, qn = 0, qh = 0;
+    if (on)
+    {
+        const PortRec &pr = s.ports[sr.port0 + lane];
+        link = pr.in_link;
+        qn = pr.q_size;
+        qh = pr.q_head;
+        if (link >= 0)
+        {
+            n2 = gt >= 2 ? msg_count(s, gt - 2, link) : 0;
+            n1 = gt >= 1 ? msg_count(s, gt - 1, link) : 0;
+        }
+    }
+    // its world does not run this slot; or no frame arriving and every queue empty: nothing to do
+    // (its link messages of this slot stay unwritten, and a stale tag reads as an empty message)
+    if (gt < next || !__any_sync(FULL, (n2 | n1 | qn) != 0))
+        return false;
+#ifdef TB_PROFILE
+    unsigned long long sp0 = globaltimer();
+#endif
+    SwCtx x;
+    x.s = &s;
+    x.wd = &s.worlds[sr.world];
+    x.sr = &sr;
+    x.sw = sw;
+    x.ports = s.ports + sr.port0;
+    x.scratch = (size_t)sw * s.kmax * 2 * MAX_TX;
+    x.t = gt - t0;
+    x.gt = gt;
+    x.spray = x.wd->spray != 0;
+    SwCounts c{};
+    int incl = n2 + n1;
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o)
+            incl += v;
+    }
+    const int total = __shfl_sync(FULL, incl, 31), first = incl - n2 - n1;
+    sh.raw2[lane] = n2;
+    sh.raw1[lane] = n1;
+    sh.link[lane] = link;
+    sh.cnt[lane] = 0;
+    bool act;
+    if (total <= sh.cap)
+    {
+        uint32_t *key = sh.key(), *mem = sh.mem();
+        uint16_t *src = sh.src();
+        uint8_t *out = sh.out();
+        const int64_t S0 = x.t * SLOT_PS, E0 = S0 + SLOT_PS;
+        // each staged frame's port (5 bits) and place in its message (9 bits, 1: of msg[t-1])
+        for (int j = 0; j < n2 + n1; j++)
+            src[first + j] = (uint16_t)(j < n2 ? lane << 10 | j : lane << 10 | 0x200 | (j - n2));
+        if (lane == 0)
+            sh.tied = 0;
+        // the queue's next frames, which the slot starts (a slot sends 8 full frames), into L1
+        if (on && qn)
+        {
+            const Frame *ring = s.port_ring + (size_t)(sr.port0 + lane) * s.ring;
+            for (int j = 0; j < 9 && j < qn; j++)
+                prefetch_l1(&ring[qh + j < s.ring ? qh + j : qh + j - s.ring]);
+        }
+        __syncwarp();
+        // the frames: copied, their place in the window
+        for (int i = lane; i < total; i += 32)
+        {
+            const int v = src[i], q = v >> 10, l = sh.link[q];
+            const bool m1 = v & 0x200;
+            Frame f;
+            frame_load_link(f, msg_frames(s, m1 ? gt - 1 : gt - 2, l) + (v & 0x1FF));
+            frame_copy(&sh.fr()[i], &f);
+            const bool in = m1 ? f.ts < E0 : f.ts >= S0;
+            c.pk += in;
+            uint32_t ky = ~0u;
+            if (in)
+            {
+                ky = (uint32_t)(f.ts - S0);
+                if (x.spray)
+                {
+                    const int ep = x.wd->n_fail ? epoch_of(*x.wd, f.ts) : 0;
+                    const bool draws = !port_down(*x.wd, sr.local, q, ep) && routes_to(*x.wd, sr.local, f.dst, ep) > 0;
+                    ky = ky << 12 | (uint32_t)(2047 - f.len) << 1 | (draws ? 0u : 1u);
+                }
+            }
+            key[i] = ky;
+        }
+        if (lane < 4 && total + lane < SwShared::pad4(total))
+            key[total + lane] = ~0u; // (the draws' scan reads whole fours)
+        __syncwarp();
+#ifdef TB_PROFILE
+        unsigned long long sp2 = globaltimer();
+        if (lane == 0)
+            atomicAdd(&s.ctl->prof_phase[11], sp2 - sp0);
+#endif
+        if (x.spray)
+        {
+            sw_spray_staged(x, sh, lane, total, first, first + n2, g_rng_ahead, c.ties);
+            __syncwarp();
+        }
+#ifdef TB_PROFILE
+        unsigned long long sp3 = globaltimer();
+        if (lane == 0)
+            atomicAdd(&s.ctl->prof_phase[12], sp3 - sp2);
+#endif
+        // each frame's egress port
+        for (int i = lane; i < total; i += 32)
+        {
+            int e = -1;
+            if (key[i] != ~0u)
+            {
+                e = sw_egress_for(x, sh.fr()[i], src[i] >> 10, x.spray ? out[i] : 0);
+                if (e < 0)
+                    c.drops++;
+                else
+                    atomicAdd(&sh.cnt[e], 1);
+            }
+            out[i] = (uint8_t)e;
+        }
+        __syncwarp();
+        const int n = sh.cnt[lane];
+        int ei = n;
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int v = __shfl_up_sync(FULL, ei, o);
+            if (lane >= o)
+                ei += v;
+        }
+        const int base = ei - n, kept = __shfl_sync(FULL, ei, 31);
+        sh.base[lane] = base;
+        __syncwarp();
+        // by egress port (in any order), then each to its place among its port's
+        for (int i = lane; i < total; i += 32)
+        {
+            const int e = (int8_t)out[i];
+            if (e >= 0)
+                mem[sh.base[e] + atomicSub(&sh.cnt[e], 1) - 1] = (x.spray ? key[i] >> 12 : key[i]) << 9 | (uint32_t)i;
+        }
+        sh.raw2[lane] = n;
+        __syncwarp();
+        for (int j = lane; j < kept; j += 32)
+        {
+            const uint32_t v = mem[j];
+            const int e = out[v & 511], b = sh.base[e], m = sh.raw2[e];
+            int rank = 0, same = 0;
+            for (int i = b; i < b + m; i++)
+            {
+                const uint32_t u = mem[i];
+                rank += u < v;
+                same += u >> 9 == v >> 9;
+            }
+            key[b + rank] = v;
+            if (same > 1)
+                atomicOr(&sh.tied, 1u << e);
+        }
+        __syncwarp();
+        if (sh.tied >> lane & 1)
+            sw_order_ties(sh, key + base, n, c.ties);
+#ifdef TB_PROFILE
+        unsigned long long sp1 = globaltimer();
+        if (lane == 0)
+            atomicAdd(&s.ctl->prof_phase[6], sp1 - sp0);
+#endif
+        __syncwarp();
+        act = on && sw_egress_staged(x, sh, lane, key + base, n, c);
+#ifdef TB_PROFILE
+        __syncwarp();
+        if (lane == 0)
+            atomicAdd(&s.ctl->prof_phase[7], globaltimer() - sp1);
+#endif
+    }
+    else
+    {
+        __syncwarp();
+        act = switch_unstaged(x, sh, lane, c);
+    }
+    __syncwarp();
+    // warp totals, one atomic each
+    c.pk = __reduce_add_sync(FULL, c.pk);
+    c.drops = __reduce_add_sync(FULL, c.drops);
+    c.marks = __reduce_add_sync(FULL, c.marks);
+    c.ovf = __reduce_add_sync(FULL, c.ovf);
+    c.ties = __reduce_add_sync(FULL, c.ties);
+    if (lane == 0)
+    {
+        ev_add(s, sr.world, EV_SW_PKT, c.pk);
+        ev_add(s, sr.world, EV_DROPS, c.drops);
+        ev_add(s, sr.world, EV_MARKS, c.marks);
+        ev_add(s, sr.world, EV_OVF_TX, c.ovf);
+        ev_add(s, sr.world, EV_TIES, c.ties);
+        ties += c.ties;
+    }
+    return __any_sync(FULL, act);
+}
+
+// MIN_BLOCKS: the register budget. Separate instantiations, chosen per launch.
+template <int MIN_BLOCKS>
 __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(Sim s, int max_slots_per_launch, int host_lanes, int stage_cap)
 {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -697,7 +606,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
     const int gwarp = blockIdx.x * WARPS_PER_BLOCK + warp, nwarps = gridDim.x * WARPS_PER_BLOCK;
     const int host_units = (s.H + host_lanes - 1) / host_lanes;
     const int units = host_units + s.S;
-    SwShared &sh = *sw_shared_at(dyn_smem + (size_t)warp * sw_shared_bytes(stage_cap, PORT_LOCAL), stage_cap); // the warp's scratch
+    SwShared &sh = *sw_shared_at(dyn_smem + (size_t)warp * sw_shared_bytes(stage_cap), stage_cap); // the warp's scratch
     __syncwarp();
     SlotCtl *ctl = s.ctl;
     volatile SlotCtl *vc = ctl;
@@ -726,7 +635,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
             else
             {
                 const int sw = u - host_units;
-                if (switch_step<PORT_LOCAL>(s, sw, t, lane, sh, ties) && lane == 0)
+                if (switch_step(s, sw, t, lane, sh, ties) && lane == 0)
                     atomicOr(&s.wctl[s.sws[sw].world].act, 1u);
             }
 #ifdef TB_PROFILE
@@ -884,13 +793,13 @@ __global__ void free_open(Sim s, unsigned budget)
     }
 }
 
-template <bool PORT_LOCAL, int MIN_BLOCKS>
+template <int MIN_BLOCKS>
 __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(Sim s, int host_lanes, int stage_cap)
 {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gwarp = blockIdx.x * WARPS_PER_BLOCK + warp, nwarps = gridDim.x * WARPS_PER_BLOCK;
-    SwShared &sh = *sw_shared_at(dyn_smem + (size_t)warp * sw_shared_bytes(stage_cap, PORT_LOCAL), stage_cap); // the warp's scratch
+    SwShared &sh = *sw_shared_at(dyn_smem + (size_t)warp * sw_shared_bytes(stage_cap), stage_cap); // the warp's scratch
     __syncwarp();
     const unsigned FULL = 0xffffffffu;
     long long idle = 0;
@@ -924,7 +833,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
                 host_unit<MIN_BLOCKS == MIN_BLOCKS_MANY>(s, v, min(host_lanes, wd.host0 + wd.H1 - v), t, lane, sh, ties,
                                                          &s.ctl->flows_done);
             }
-            else if (switch_step<PORT_LOCAL>(s, v - s.H, t, lane, sh, ties) && lane == 0)
+            else if (switch_step(s, v - s.H, t, lane, sh, ties) && lane == 0)
                 atomicOr(&s.wctl[w].act, 1u);
             __syncwarp();
             if (lane == 0)
@@ -957,40 +866,31 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
 }
 
 // dynamic shared memory of a block: one switch scratch (with its staging area) per warp
-static size_t smem_bytes(int stage_cap, bool port_local) { return sw_shared_bytes(stage_cap, port_local) * WARPS_PER_BLOCK; }
+static size_t smem_bytes(int stage_cap) { return sw_shared_bytes(stage_cap) * WARPS_PER_BLOCK; }
 
-// the instantiation of a launch shape: several hosts per warp, one host per warp, one host per
-// warp with port-local switch egress; each with the grid barrier or without (F_*: batches)
+// the instantiation of a launch shape: several hosts per warp or one host per warp; each with the
+// grid barrier or without (F_*: batches)
 enum
 {
     K_MANY,
     K_ONE,
-    K_ONE_PL,
     F_MANY,
     F_ONE,
-    F_ONE_PL,
     K_N
 };
-static int kind_of(int host_lanes, bool port_local, bool free = false)
-{
-    return (host_lanes > 1 ? K_MANY : port_local ? K_ONE_PL : K_ONE) + (free ? F_MANY : 0);
-}
+static int kind_of(int host_lanes, bool free = false) { return (host_lanes > 1 ? K_MANY : K_ONE) + (free ? F_MANY : 0); }
 static const void *kernel_of(int k)
 {
     switch (k)
     {
     case K_MANY:
-        return (const void *)slot_kernel<false, MIN_BLOCKS_MANY>;
+        return (const void *)slot_kernel<MIN_BLOCKS_MANY>;
     case K_ONE:
-        return (const void *)slot_kernel<false, MIN_BLOCKS_ONE>;
-    case K_ONE_PL:
-        return (const void *)slot_kernel<true, MIN_BLOCKS_ONE>;
+        return (const void *)slot_kernel<MIN_BLOCKS_ONE>;
     case F_MANY:
-        return (const void *)free_kernel<false, MIN_BLOCKS_MANY>;
-    case F_ONE:
-        return (const void *)free_kernel<false, MIN_BLOCKS_ONE>;
+        return (const void *)free_kernel<MIN_BLOCKS_MANY>;
     default:
-        return (const void *)free_kernel<true, MIN_BLOCKS_ONE>;
+        return (const void *)free_kernel<MIN_BLOCKS_ONE>;
     }
 }
 
@@ -1000,8 +900,7 @@ static bool smem_attr(int k)
     if (!tried[k])
     {
         tried[k] = true;
-        const bool pl = k == K_ONE_PL || k == F_ONE_PL;
-        ok[k] = cudaFuncSetAttribute(kernel_of(k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(SW_STAGE_MAX, pl)) == cudaSuccess;
+        ok[k] = cudaFuncSetAttribute(kernel_of(k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(SW_STAGE_MAX)) == cudaSuccess;
     }
     return ok[k];
 }
@@ -1009,35 +908,34 @@ static bool smem_attr(int k)
 // The preferred shared-memory carveout, in percent of the SM's maximum: the shared memory of the
 // blocks a launch puts on one SM and no more, so that the rest of the SM's unified L1 / shared
 // memory is L1, where the units' records, ring heads and prefetched lines stay between slots.
-static int carveout[K_N] = {-1, -1, -1, -1, -1, -1}; // the last ones set (-1: none)
+static int carveout[K_N] = {-1, -1, -1, -1}; // the last ones set (-1: none)
 static void set_carveout(int k, int pct)
 {
     if (pct != carveout[k] && cudaFuncSetAttribute(kernel_of(k), cudaFuncAttributePreferredSharedMemoryCarveout, pct) == cudaSuccess)
         carveout[k] = pct;
 }
 
-int slot_kernel_blocks_per_sm(int stage_cap, bool port_local, int host_lanes, bool free)
+int slot_kernel_blocks_per_sm(int stage_cap, int host_lanes, bool free)
 {
     int n = 0;
-    port_local = port_local && host_lanes == 1;
-    const int k = kind_of(host_lanes, port_local, free);
+    const int k = kind_of(host_lanes, free);
     if (stage_cap < 1 || stage_cap > SW_STAGE_MAX || !smem_attr(k))
         return 0;
     set_carveout(k, 100); // (occupancy with all of the shared memory)
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel_of(k), WARPS_PER_BLOCK * 32, smem_bytes(stage_cap, port_local)) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel_of(k), WARPS_PER_BLOCK * 32, smem_bytes(stage_cap)) != cudaSuccess)
         return 0;
     return n;
 }
 
 // a cooperative launch of kernel kind k (all its blocks resident: the waits need it)
-static int launch_kind(int k, void **args, int grid, int stage_cap, bool port_local, cudaStream_t stream)
+static int launch_kind(int k, void **args, int grid, int stage_cap, cudaStream_t stream)
 {
     int dev = 0, sms = 1, max_smem = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     const long long per_sm = (grid + sms - 1) / sms;
-    const size_t bytes = smem_bytes(stage_cap, port_local);
+    const size_t bytes = smem_bytes(stage_cap);
     const long long need = per_sm * (long long)(bytes + 2048); // (+ the block's reserved and static shared memory)
     set_carveout(k, (int)std::min<long long>(100, (need * 100 + max_smem - 1) / max_smem));
     cudaError_t e = cudaLaunchCooperativeKernel(kernel_of(k), dim3(grid), dim3(WARPS_PER_BLOCK * 32), args, bytes, stream);
@@ -1051,20 +949,18 @@ static int launch_kind(int k, void **args, int grid, int stage_cap, bool port_lo
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-int launch_slots(const Sim &s, int grid, int max_slots_per_launch, int host_lanes, int stage_cap, bool port_local, cudaStream_t stream)
+int launch_slots(const Sim &s, int grid, int max_slots_per_launch, int host_lanes, int stage_cap, cudaStream_t stream)
 {
-    port_local = port_local && host_lanes == 1; // (several hosts per warp: the plain egress)
-    const int k = kind_of(host_lanes, port_local);
+    const int k = kind_of(host_lanes);
     if (!smem_attr(k) || stage_cap < 1 || stage_cap > SW_STAGE_MAX)
         return (int)cudaErrorInvalidValue;
     void *args[] = {(void *)&s, (void *)&max_slots_per_launch, (void *)&host_lanes, (void *)&stage_cap};
-    return launch_kind(k, args, grid, stage_cap, port_local, stream);
+    return launch_kind(k, args, grid, stage_cap, stream);
 }
 
-int launch_free(const Sim &s, int grid, int slots_per_world, int host_lanes, int stage_cap, bool port_local, cudaStream_t stream)
+int launch_free(const Sim &s, int grid, int slots_per_world, int host_lanes, int stage_cap, cudaStream_t stream)
 {
-    port_local = port_local && host_lanes == 1;
-    const int k = kind_of(host_lanes, port_local, true);
+    const int k = kind_of(host_lanes, true);
     if (!smem_attr(k) || stage_cap < 1 || stage_cap > SW_STAGE_MAX || !s.unit_list || !s.unit_done || !s.w_units || slots_per_world < 1)
         return (int)cudaErrorInvalidValue;
     const int n = std::max(s.n_list, s.W);
@@ -1073,21 +969,21 @@ int launch_free(const Sim &s, int grid, int slots_per_world, int host_lanes, int
     if (e != cudaSuccess)
         return (int)e;
     void *args[] = {(void *)&s, (void *)&host_lanes, (void *)&stage_cap};
-    return launch_kind(k, args, grid, stage_cap, port_local, stream);
+    return launch_kind(k, args, grid, stage_cap, stream);
 }
 
 // A launch as a CUDA graph: the launch is captured once per shape, slot count and unit list and
 // replayed as a graph; where capturing or instantiating fails, plain launches follow for good.
 // free: the batch kernel without a grid barrier (launch_free), with its opening kernel.
-int launch_slots_graph(SlotGraph &g, const Sim &s, int grid, int max_slots_per_launch, int host_lanes, int stage_cap, bool port_local,
+int launch_slots_graph(SlotGraph &g, const Sim &s, int grid, int max_slots_per_launch, int host_lanes, int stage_cap,
                        cudaStream_t stream, bool free)
 {
-    const unsigned long long key[9] = {(unsigned long long)grid, (unsigned long long)max_slots_per_launch, (unsigned long long)host_lanes,
-                                       (unsigned long long)stage_cap, (unsigned long long)port_local, (unsigned long long)(uintptr_t)s.unit_list,
+    const unsigned long long key[8] = {(unsigned long long)grid, (unsigned long long)max_slots_per_launch, (unsigned long long)host_lanes,
+                                       (unsigned long long)stage_cap, (unsigned long long)(uintptr_t)s.unit_list,
                                        (unsigned long long)s.n_list, (unsigned long long)s.max_slots, (unsigned long long)free};
     auto go = [&]() {
-        return free ? launch_free(s, grid, max_slots_per_launch, host_lanes, stage_cap, port_local, stream)
-                    : launch_slots(s, grid, max_slots_per_launch, host_lanes, stage_cap, port_local, stream);
+        return free ? launch_free(s, grid, max_slots_per_launch, host_lanes, stage_cap, stream)
+                    : launch_slots(s, grid, max_slots_per_launch, host_lanes, stage_cap, stream);
     };
     if (g.broken)
         return go();
