@@ -35,9 +35,20 @@ __device__ __forceinline__ unsigned long long globaltimer()
     return t;
 }
 
-// The barrier's generation word. Cross-SM data (link messages, the controller) is read from L2
-// (ld.cg, volatile, atomics) and every entity's private state stays on its SM, so the wait needs
-// no acquire load, which would invalidate the L1 that holds the entities' records.
+// The barriers' words. Cross-SM data (link messages, the controller) is read from L2 (ld.cg,
+// volatile, atomics) and every entity's private state stays on its SM, so a wait needs no acquire,
+// and an arrival only a release: a full fence (__threadfence) on either side would also invalidate
+// the SM's L1, which holds the entities' records, for every warp of the SM in every slot.
+__device__ __forceinline__ unsigned add_release(unsigned *p, unsigned v)
+{
+    unsigned o;
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
+    return o;
+}
+__device__ __forceinline__ void st_release(int64_t *p, int64_t v)
+{
+    asm volatile("st.release.gpu.global.s64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ unsigned ld_gen(const unsigned *p)
 {
     unsigned v;
@@ -653,14 +664,11 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
             blk_alive = 0;
             // grid barrier: the last block to arrive ends the slot and releases the others
             g = ld_gen(&ctl->gen);
-            __threadfence();
-            unsigned arrived = atomicAdd(&ctl->arrive, 1u) + 1;
-            blk_last = arrived == gridDim.x;
+            blk_last = add_release(&ctl->arrive, 1u) + 1 == gridDim.x;
         }
         __syncthreads();
         if (blk_last)
         {
-            __threadfence();
             // every world's next slot: finished worlds stop; a world where nothing was sent in
             // this or the previous slot skips to its earliest wake-up
             for (int w = threadIdx.x; w < s.W; w += blockDim.x)
@@ -709,8 +717,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
                 vc->prof_host_max = 0;
                 vc->prof_sw_max = 0;
 #endif
-                __threadfence();
-                atomicAdd(&ctl->gen, 1u);
+                add_release(&ctl->gen, 1u);
             }
         }
         else if (threadIdx.x == 0)
@@ -728,8 +735,6 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
                 __nanosleep(64);
             }
         }
-        if (threadIdx.x == 0)
-            __threadfence();
         __syncthreads();
     }
 }
@@ -751,7 +756,6 @@ __device__ void world_close(const Sim &s, int w, int64_t t)
 {
     WorldCtl *wc = &s.wctl[w];
     volatile WorldCtl *vw = wc;
-    __threadfence();
     const unsigned cur = atomicExch(&wc->act, 0u), prev = vw->prev;
     const unsigned long long wake = atomicExch(&wc->wake, (unsigned long long)INT64_MAX);
     vw->prev = cur;
@@ -773,8 +777,7 @@ __device__ void world_close(const Sim &s, int w, int64_t t)
     vw->budget = budget;
     vw->next = nx;
     vw->arrive = 0;
-    __threadfence();
-    vw->run = (nx == INT64_MAX || budget == 0) ? RUN_PARKED : nx;
+    st_release(&wc->run, (nx == INT64_MAX || budget == 0) ? RUN_PARKED : nx);
 }
 
 // before a launch: every world runs from its next slot with a budget; every unit has done nothing
@@ -825,7 +828,6 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
             if (done == t)
                 continue; // (done; its world's other units are not)
             ran = true;
-            __threadfence(); // (what the world's units wrote in its last slot, before `run` moved)
             unsigned ties = 0;
             if (host)
             {
@@ -839,8 +841,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
             if (lane == 0)
             {
                 s.unit_done[i] = t;
-                __threadfence();
-                if (atomicAdd(&s.wctl[w].arrive, 1u) + 1 == __ldcg(&s.wctl[w].units))
+                if (add_release(&s.wctl[w].arrive, 1u) + 1 == __ldcg(&s.wctl[w].units))
                     world_close(s, w, t);
             }
             __syncwarp();

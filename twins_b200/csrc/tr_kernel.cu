@@ -11,6 +11,15 @@ namespace tr
 
 constexpr long long BARRIER_SPIN_LIMIT = 1ll << 22; // polls of ~64 ns: a quarter of a second or more
 
+// What crosses SMs (frames, bucket tags, tail nodes, the controller) is read from L2, and an entity's
+// own records stay on its SM: the barrier releases what its block wrote, and needs no full fence
+// (__threadfence), which would invalidate the L1 that holds the records in every slot.
+__device__ __forceinline__ unsigned add_release(unsigned *p, unsigned v)
+{
+    unsigned o;
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
+    return o;
+}
 __device__ __forceinline__ unsigned ld_volatile(const unsigned *p) { return *(const volatile unsigned *)p; }
 #ifdef TR_PROFILE
 __device__ __forceinline__ unsigned long long gtimer()
@@ -102,15 +111,13 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32) rdma_slot_kernel(RSim s, int 
         if (threadIdx.x == 0)
         {
             g = ld_volatile(&ctl->gen);
-            __threadfence();
-            blk_last = atomicAdd(&ctl->arrive, 1u) + 1 == gridDim.x;
+            blk_last = add_release(&ctl->arrive, 1u) + 1 == gridDim.x;
         }
         __syncthreads();
         if (threadIdx.x == 0)
         {
             if (blk_last)
             {
-                __threadfence();
                 const unsigned act = atomicExch(&ctl->activity, 0u);
                 const unsigned long long wake = atomicExch(&ctl->next_wake, ~0ull);
                 const unsigned done = atomicAdd(&ctl->flows_done, 0u);
@@ -125,8 +132,7 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32) rdma_slot_kernel(RSim s, int 
                 s.ev[EV_PROF_LANE_EV] += atomicExch(&s.ev[EV_PROF_LANE_EV_SLOT], 0ull);
 #endif
                 vc->arrive = 0;
-                __threadfence();
-                atomicAdd(&ctl->gen, 1u);
+                add_release(&ctl->gen, 1u);
             }
             else
             {
@@ -143,7 +149,6 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32) rdma_slot_kernel(RSim s, int 
                     __nanosleep(64);
                 }
             }
-            __threadfence();
         }
         __syncthreads();
     }

@@ -1953,10 +1953,11 @@ TR_HD bool switch_slot(const RSim &s, int x, int64_t t, const SwWork &w, int lan
 // After every entity ran slot t: the run ends when every flow is done or at the stop time; a slot
 // in which nothing was sent or held goes on at the earliest host event or frame arrival; nothing
 // left at all ends the run (quiescence). (reference: slot_end, src/rdma/rstep.cuh:3451-3577)
-// (activity, next_wake and flows_done: the entities' sums of the slot, read by the caller)
+// (activity, next_wake and flows_done: the entities' sums of the slot, read by the caller; the
+// controller is another SM's in the next slot: no L1 copy of it is read)
 TR_HD void slot_close(const RSim &s, int64_t t, unsigned activity, unsigned long long next_wake, unsigned flows_done)
 {
-    RCtl &c = *s.ctl;
+    volatile RCtl &c = *s.ctl;
     if (flows_done >= (unsigned)s.F || t + 1 >= s.max_slots)
         c.finished = 1;
     s.pend[t % s.pend_n] = 0;
@@ -1976,7 +1977,7 @@ TR_HD void slot_close(const RSim &s, int64_t t, unsigned activity, unsigned long
             c.finished = 1;
     }
     c.slot = next;
-    c.slots_run++;
+    c.slots_run = c.slots_run + 1;
 }
 
 } // namespace tr
