@@ -22,10 +22,11 @@ namespace tb
 {
 
 constexpr int WARPS_PER_BLOCK = TB_WARPS_PER_BLOCK;
-// resident blocks per SM that each instantiation's register budget allows: 4 for several hosts
-// per warp (with the smaller staging areas, four blocks fit an SM), 2 for one host per warp (two
-// blocks at most fit with its staging areas; more registers spare the host's event loop spills)
-constexpr int MIN_BLOCKS_MANY = 4, MIN_BLOCKS_ONE = 2;
+// resident blocks per SM that each instantiation's register budget allows. Several hosts per warp: 3
+// (168 registers: with 4 blocks, 128 registers, the connection core spills and 96 k=8 worlds take
+// 186 ms, with 3 163 ms). One host per warp: 2, and up to 255 registers (with 3 blocks the event loop
+// spills: 12 leaf-spine worlds 297 / 233 ms, 96 k=8 worlds 281 / 252 ms).
+constexpr int MIN_BLOCKS_MANY = 3, MIN_BLOCKS_ONE = 2;
 constexpr long long BARRIER_SPIN_LIMIT = 1ll << 22; // polls of >= 64 ns: several seconds
 
 __device__ __forceinline__ unsigned long long globaltimer()

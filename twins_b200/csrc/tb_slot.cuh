@@ -170,6 +170,14 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
     const int pe = hr.pend_end;
     Frame p;
     bool have_p = false; // p holds the next arrival
+    // the next application event and its start (at or after E0: none this slot)
+    int pm = -1;
+    int64_t pst = INT64_MAX;
+    auto next_pend = [&]() {
+        pm = pn < pe ? s.pend_msg[pn] : -1;
+        pst = pm >= 0 ? s.msgs[pm].start : INT64_MAX;
+    };
+    next_pend();
     for (;;)
     {
         int64_t tr = INT64_MAX, td = INT64_MAX, tp = INT64_MAX;
@@ -190,14 +198,8 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
             tr = p.ts;
         if (c.di < c.nd)
             td = c.due[c.di].at;
-        int pm = -1;
-        if (pn < pe)
-        {
-            pm = s.pend_msg[pn];
-            int64_t st = s.msgs[pm].start;
-            if (st < E0)
-                tp = st;
-        }
+        if (pst < E0)
+            tp = pst;
         int64_t now = tr < td ? tr : td;
         now = now < tp ? now : tp;
         if (now == INT64_MAX)
@@ -209,8 +211,9 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
         TB_PHASE(8)
         if (now == tp)
         {
-            pn++;
             app_event(c, hr, act_snd, pm, now);
+            pn++;
+            next_pend();
             TB_PHASE(10)
             continue;
         }
@@ -291,12 +294,8 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
         }
         hr.n_rcv = k;
     }
-    if (pn < pe)
-    {
-        int64_t st = s.msgs[s.pend_msg[pn]].start;
-        if (st < next)
-            next = st;
-    }
+    if (pst < next)
+        next = pst;
     hr.wake = nic.size > 0 ? t + 1 : (next == INT64_MAX ? INT64_MAX : next / SLOT_PS);
     *wake = hr.wake;
     TB_PHASE(4)

@@ -47,15 +47,20 @@ TB_HD uint32_t sent_list_cap(uint64_t segs)
     return (uint32_t)((n + 7) & ~7ull);
 }
 
-// the sending side of a connection (TcpSocketBase, TcpTxBuffer, the congestion control)
-struct SndRec
+// The sending side of a connection (TcpSocketBase, TcpTxBuffer, the congestion control). A record has
+// a core, which every event of its connection works on in registers (tb_tcp.cuh: Snd, loaded when the
+// event begins and stored when it ends, in 16-byte words), and the rest, which few events touch and
+// which stays in memory. The core begins with what never changes, which is not stored back.
+constexpr int REC_FIXED = 48; // the bytes of both records' cores that never change
+struct alignas(16) SndCore
 {
     // read-only
+    uint64_t it_off;
     int world, src_local, dst_local;
     uint32_t hash_data, hash_ack;
     int m_first, m_cnt; // messages (global ids, consecutive)
     uint32_t it_cap;    // sent-list / RTT-history ring capacity
-    uint64_t it_off;
+    uint32_t pad0[2];
     // application and socket
     int m_due, m_wr, m_dn;
     uint8_t st, cong, fin, fin_on;
@@ -65,34 +70,42 @@ struct SndRec
     uint32_t sack_b, lost_b, rtx_b, cand_b, sack_n, cand_lo, hisack; // the sent list's byte counters, sacked items, first-candidate bound, highest sack
     uint8_t sack_seen, recover_active, first_partial, cwnd_limited;
     uint32_t recover, cwnd_cnt, ack_rem;
-    // TcpCubic
-    uint32_t cub_cnt, cub_lastmax, cub_origin, cub_endseq, cub_samples, cub_ackcnt, cub_tcpcwnd;
-    uint8_t cub_found, s_ce, ecn_s, next_seq_flag;
-    double cub_k;
-    int64_t cub_delaymin, cub_epoch, cub_roundstart, cub_lastack, cub_currrtt;
+    uint8_t syn_tries, s_ce, ecn_s, next_seq_flag;
     // ECN / DCTCP
+    uint32_t acked_total, acked_ecn, next_seq;
     int64_t ecn_echo_seq, ecn_cwr_seq;
     double alpha;
-    uint32_t acked_total, acked_ecn, next_seq;
-    uint8_t syn_tries, pad0[3];
     // RTT and timers
     int64_t srtt, rttvar, rto, rto_at, timing_time, syn_at;
+};
+struct SndRec : SndCore
+{
+    // TcpCubic
+    uint32_t cub_cnt, cub_lastmax, cub_origin, cub_endseq, cub_samples, cub_ackcnt, cub_tcpcwnd;
+    uint8_t cub_found, pad1[3];
+    double cub_k;
+    int64_t cub_delaymin, cub_epoch, cub_roundstart, cub_lastack, cub_currrtt;
     Chain rchain; // the retransmission (or SYN) timer's
     Chain schain; // the deferred SendPendingData's
 };
 
 // the receiving side (TcpRxBuffer, delayed ACKs, DCTCP's CE state, the closing states)
-struct RcvRec
+struct alignas(16) RcvCore
 {
+    uint64_t oo_off;
     int world, src_local, dst_local;
     uint32_t hash_ack;
     uint32_t oo_cap;
-    uint64_t oo_off;
     uint32_t bytes;             // the connection's bytes (all its messages)
+    uint32_t pad0[4];
     uint8_t fin_on, up, est, st;
-    int64_t fin_seq, synack_t, srtt, rttvar, last_at, frx_at, syn_at, delack_at, ecn_ce_seq;
     uint32_t rcv_nxt, ooo_n, ooo_h, prior_rcv_nxt;
-    uint8_t last_n, syn_n, delack_count, ce_state, prior_flag, reserved, ecn_r, pad0;
+    uint8_t last_n, syn_n, delack_count, ce_state, prior_flag, reserved, ecn_r, pad1;
+    uint32_t pad2;
+    int64_t fin_seq, synack_t, srtt, rttvar, last_at, frx_at, syn_at, delack_at, ecn_ce_seq, pad3;
+};
+struct RcvRec : RcvCore
+{
     Chain dchain; // delayed ACK, SYN-ACK retransmission, LastAckTimeout
     Chain fchain; // the FIN+ACK's own retransmission
 };

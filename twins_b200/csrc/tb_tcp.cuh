@@ -6,6 +6,8 @@
 #pragma once
 #include "tb_egress.cuh"
 
+#include <cstddef>
+
 namespace tb
 {
 
@@ -34,6 +36,29 @@ struct HostCtx
     unsigned retx, rtos, ovf, done;
     unsigned long long pkts, snd_pkts;
 };
+
+// A connection's record while an event works on it: its core in registers (a record worked on in
+// place is read and written through memory field by field, since the compiler cannot tell it from
+// the rings and frames the event stores), the rest of it behind `rec`.
+struct Snd : SndCore
+{
+    SndRec *rec;
+    TB_D explicit Snd(SndRec &r) : SndCore(r), rec(&r) {}
+    TB_D void store() const { store_core(rec, this, sizeof(SndCore)); }
+    // the words of a core that change, back to its record
+    TB_D static void store_core(void *to, const void *from, size_t bytes)
+    {
+        memcpy((char *)to + REC_FIXED, (const char *)from + REC_FIXED, bytes - REC_FIXED);
+    }
+};
+struct Rcv : RcvCore
+{
+    RcvRec *rec;
+    TB_D explicit Rcv(RcvRec &r) : RcvCore(r), rec(&r) {}
+    TB_D void store() const { Snd::store_core(rec, this, sizeof(RcvCore)); }
+};
+static_assert(offsetof(SndCore, m_due) == REC_FIXED && offsetof(RcvCore, fin_on) == REC_FIXED && sizeof(SndCore) % 16 == 0 && sizeof(RcvCore) % 16 == 0,
+              "cores move as 16-byte words");
 
 // a timer armed during the slot that falls due before its end joins the slot's timers, after the
 // ones of its time already there (reference: due_insert, src/step.cuh:342-360)
@@ -71,11 +96,11 @@ TB_D void to_device(HostCtx &c, int f, uint8_t flags, uint32_t num, uint16_t wir
     fr.ch = c.ech;
     c.nic.enqueue(fr, now);
 }
-TB_D void emit_snd(HostCtx &c, int f, const SndRec &S, uint8_t flags, uint32_t num, uint16_t wire_len, int64_t now)
+TB_D void emit_snd(HostCtx &c, int f, const SndCore &S, uint8_t flags, uint32_t num, uint16_t wire_len, int64_t now)
 {
     to_device(c, f, flags, num, wire_len, false, S.hash_data, S.dst_local, now);
 }
-TB_D void emit_rcv(HostCtx &c, int f, const RcvRec &R, uint8_t flags, uint32_t ack, uint16_t len, int64_t now)
+TB_D void emit_rcv(HostCtx &c, int f, const RcvCore &R, uint8_t flags, uint32_t ack, uint16_t len, int64_t now)
 {
     to_device(c, f, flags, ack, len, true, R.hash_ack, R.src_local, now);
 }
@@ -89,7 +114,7 @@ enum AckEcho
     ECHO_FORCE,
     ECHO_NEVER
 };
-TB_D void rcv_ack(HostCtx &c, int f, RcvRec &R, uint32_t ack, AckEcho echo, int64_t now)
+TB_D void rcv_ack(HostCtx &c, int f, RcvCore &R, uint32_t ack, AckEcho echo, int64_t now)
 {
     bool ece = echo == ECHO_FORCE;
     if (echo == ECHO_AS_STATE && (R.ecn_r == E_CE_RCVD || R.ecn_r == E_SENDING_ECE))
@@ -125,12 +150,12 @@ enum : uint8_t
 
 struct SentList
 {
-    SndRec &S;
+    SndCore &S;
     uint32_t *start;
     uint32_t *fw; // flag words
     uint32_t cap;
 
-    TB_D SentList(const Sim &s, SndRec &S_) : S(S_)
+    TB_D SentList(const Sim &s, SndCore &S_) : S(S_)
     {
         start = s.it_start + S.it_off;
         fw = reinterpret_cast<uint32_t *>(s.it_fl + S.it_off);
@@ -331,8 +356,8 @@ struct SentList
 
 // bytes sent and not acknowledged; BytesInFlight = sent - (sacked + lost) + retransmitted, in
 // unsigned arithmetic as ns-3 computes it (reference: src/step.cuh:594-607)
-TB_D uint32_t sent_bytes(const SndRec &S) { return S.it_n ? S.high - S.una : 0u; }
-TB_D uint32_t inflight(const SndRec &S) { return sent_bytes(S) - (S.sack_b + S.lost_b) + S.rtx_b; }
+TB_D uint32_t sent_bytes(const SndCore &S) { return S.it_n ? S.high - S.una : 0u; }
+TB_D uint32_t inflight(const SndCore &S) { return sent_bytes(S) - (S.sack_b + S.lost_b) + S.rtx_b; }
 
 // a retransmission candidate: lost, neither retransmitted nor sacked
 TB_D uint32_t candidates(uint32_t l, uint32_t r, uint32_t k) { return l & ~r & ~k; }
@@ -341,7 +366,7 @@ TB_D uint32_t candidates(uint32_t l, uint32_t r, uint32_t k) { return l & ~r & ~
 // sacked; the highest sack moves there (reference: src/step.cuh:649-662)
 TB_D void reno_sack_one(SentList &L)
 {
-    SndRec &S = L.S;
+    SndCore &S = L.S;
     const uint32_t i = L.find(1 + S.sack_n, [](uint32_t, uint32_t, uint32_t k) { return ~k; });
     if (i >= L.n())
         return;
@@ -360,7 +385,7 @@ TB_D void head_to_lost(SentList &L)
 // src/step.cuh:687-712)
 TB_D void everything_lost(SentList &L)
 {
-    SndRec &S = L.S;
+    SndCore &S = L.S;
     // whole words: every position of a word holding a live item reads lost, neither retransmitted
     // nor sacked (its free positions too, which no read reaches before they are written)
     for (uint32_t i = 0; i < S.it_n;)
@@ -381,7 +406,7 @@ TB_D void everything_lost(SentList &L)
 // forgotten (reference: src/step.cuh:716-780)
 TB_D uint32_t ack_drop(SentList &L, uint32_t ack)
 {
-    SndRec &S = L.S;
+    SndCore &S = L.S;
     // (the walk keeps the head, the count and the flags' byte sums in registers and settles the
     // record once; an item leaving keeps its stale flag bits, which no read reaches)
     const uint32_t n = S.it_n, high = S.high;
@@ -436,7 +461,7 @@ TB_D uint32_t ack_drop(SentList &L, uint32_t ack)
 // new data beyond `high` (reference: src/step.cuh:784-834)
 TB_D bool next_to_send(const SentList &L, uint32_t *seq)
 {
-    const SndRec &S = L.S;
+    const SndCore &S = L.S;
     const uint32_t i = S.cand_b ? L.find(S.cand_lo, candidates) : L.n();
     if (i < L.n())
         L.S.cand_lo = i;
@@ -455,14 +480,14 @@ TB_D bool next_to_send(const SentList &L, uint32_t *seq)
 // IsLost(SND.UNA) (reference: src/step.cuh:838-846)
 TB_D bool first_is_lost(const SentList &L)
 {
-    const SndRec &S = L.S;
+    const SndCore &S = L.S;
     return S.sack_seen && S.una < S.hisack && L.n() && (L.flags(0) & FL_LOST);
 }
 // IsRetransmittedDataAcked(x): an item ends exactly at x, retransmitted and not sacked (reference:
 // src/step.cuh:849-869)
 TB_D bool retransmission_ends_at(const SentList &L, uint32_t x)
 {
-    const SndRec &S = L.S;
+    const SndCore &S = L.S;
     if (!L.n() || x <= S.una || x > S.high)
         return false;
     const uint32_t i = L.first_from(x) - 1; // (the item holding byte x - 1)
@@ -479,7 +504,7 @@ TB_D bool retransmission_ends_at(const SentList &L, uint32_t x)
 // src/step.cuh:874-916)
 TB_D uint32_t resend_item(SentList &L, uint32_t i, uint32_t want, unsigned &ovf)
 {
-    SndRec &S = L.S;
+    SndCore &S = L.S;
     uint32_t len = L.end(i) - L.beg(i);
     uint32_t limit = len;
     if (i + 1 < S.it_n)
@@ -511,7 +536,7 @@ TB_D uint32_t resend_item(SentList &L, uint32_t i, uint32_t want, unsigned &ovf)
 // was); a send straddling `high` is cut at `high` (reference: src/step.cuh:920-975)
 TB_D uint32_t take_segment(SentList &L, uint32_t want, uint32_t seq, bool *again, unsigned &ovf)
 {
-    SndRec &S = L.S;
+    SndCore &S = L.S;
     for (;;)
     {
         const uint32_t avail = S.tail > seq ? S.tail - seq : 0;
@@ -556,7 +581,7 @@ TB_D int64_t rto_of(int64_t srtt, int64_t rttvar)
 }
 // a measurement m: the first sets srtt = m, rttvar = m / 2; later ones move srtt by an eighth and
 // rttvar by a quarter of the difference, rounded down as ns-3's shifts round
-TB_D void rtt_update(SndRec &S, int64_t m)
+TB_D void rtt_update(SndCore &S, int64_t m)
 {
     if (S.srtt < 0)
     {
@@ -578,10 +603,10 @@ TB_D void rtt_update(SndRec &S, int64_t m)
 // (negative), so that the entry gives no sample (Karn) (reference: src/step.cuh:977-1126)
 struct RttLog
 {
-    SndRec &S;
+    SndCore &S;
     uint32_t *lo, *hi;
     int64_t *at;
-    TB_D RttLog(const Sim &s, SndRec &S_) : S(S_), lo(s.h_seq + S_.it_off), hi(s.h_end + S_.it_off), at(s.h_t + S_.it_off) {}
+    TB_D RttLog(const Sim &s, SndCore &S_) : S(S_), lo(s.h_seq + S_.it_off), hi(s.h_end + S_.it_off), at(s.h_t + S_.it_off) {}
     TB_D uint32_t slot(uint32_t j) const
     {
         const uint32_t x = S.h_head + j;
@@ -650,12 +675,12 @@ TB_D uint32_t x86_u32(double d)
     return (uint32_t)(uint64_t)(fits ? (int64_t)d : INT64_MIN);
 }
 // HyStart's round: starts now, ends when the byte after the highest sent is acknowledged
-TB_D void new_round(SndRec &S, int64_t now)
+TB_D void new_round(Snd &S, int64_t now)
 {
-    S.cub_roundstart = S.cub_lastack = now;
-    S.cub_endseq = S.st == S_EST ? S.high + 1 : 0;
-    S.cub_currrtt = INT64_MIN;
-    S.cub_samples = 0;
+    S.rec->cub_roundstart = S.rec->cub_lastack = now;
+    S.rec->cub_endseq = S.st == S_EST ? S.high + 1 : 0;
+    S.rec->cub_currrtt = INT64_MIN;
+    S.rec->cub_samples = 0;
 }
 // K = cbrt(n / C) as the host's libm pow(n / C, 1/3) gives it (a host-made table), else the device pow
 TB_D double k_of(const Sim &s, uint32_t n)
@@ -663,126 +688,126 @@ TB_D double k_of(const Sim &s, uint32_t n)
     return n < (uint32_t)s.cub_k_n ? s.cub_k_tab[n] : tb_pow((double)n / C, 1 / 3.);
 }
 // the ACKs that one more segment of window takes (ns-3's Update)
-TB_D uint32_t acks_per_segment(const Sim &s, SndRec &S, uint32_t segs, int64_t now)
+TB_D uint32_t acks_per_segment(const Sim &s, Snd &S, uint32_t segs, int64_t now)
 {
     const uint32_t w = S.cwnd / MSS;
-    S.cub_ackcnt += segs;
-    if (S.cub_epoch == INT64_MIN)
+    S.rec->cub_ackcnt += segs;
+    if (S.rec->cub_epoch == INT64_MIN)
     {
         // a new epoch: the curve's plateau is the window before the last loss, K away
-        const bool below = S.cub_lastmax > w;
-        S.cub_epoch = now;
-        S.cub_ackcnt = segs;
-        S.cub_tcpcwnd = w;
-        S.cub_k = below ? k_of(s, S.cub_lastmax - w) : 0.0;
-        S.cub_origin = below ? S.cub_lastmax : w;
+        const bool below = S.rec->cub_lastmax > w;
+        S.rec->cub_epoch = now;
+        S.rec->cub_ackcnt = segs;
+        S.rec->cub_tcpcwnd = w;
+        S.rec->cub_k = below ? k_of(s, S.rec->cub_lastmax - w) : 0.0;
+        S.rec->cub_origin = below ? S.rec->cub_lastmax : w;
     }
     // the curve one minimum RTT ahead: origin -/+ C |t - K|^3
-    const int64_t t = (int64_t)((uint64_t)now + (uint64_t)S.cub_delaymin - (uint64_t)S.cub_epoch);
-    const double ts = get_seconds(t), K = S.cub_k;
+    const int64_t t = (int64_t)((uint64_t)now + (uint64_t)S.rec->cub_delaymin - (uint64_t)S.rec->cub_epoch);
+    const double ts = get_seconds(t), K = S.rec->cub_k;
     const bool rising = ts < K;
     const uint32_t d = x86_u32(C * tb_pow(rising ? K - ts : ts - K, 3));
-    const uint32_t target = rising ? S.cub_origin - d : S.cub_origin + d;
+    const uint32_t target = rising ? S.rec->cub_origin - d : S.rec->cub_origin + d;
     uint32_t cnt = target > w ? w / (target - w) : 100 * w;
-    if (S.cub_lastmax == 0 && cnt > 20)
+    if (S.rec->cub_lastmax == 0 && cnt > 20)
         cnt = 20;
     // TCP friendliness: the window Reno would have reached on the same ACKs bounds cnt
     const uint32_t per = (w * FRIENDLY) >> 3;
-    if (S.cub_ackcnt > per)
+    if (S.rec->cub_ackcnt > per)
     {
-        const uint32_t k = (S.cub_ackcnt - 1) / per;
-        S.cub_ackcnt -= k * per;
-        S.cub_tcpcwnd += k;
+        const uint32_t k = (S.rec->cub_ackcnt - 1) / per;
+        S.rec->cub_ackcnt -= k * per;
+        S.rec->cub_tcpcwnd += k;
     }
-    if (S.cub_tcpcwnd > w)
+    if (S.rec->cub_tcpcwnd > w)
     {
-        const uint32_t bound = w / (S.cub_tcpcwnd - w);
+        const uint32_t bound = w / (S.rec->cub_tcpcwnd - w);
         cnt = cnt < bound ? cnt : bound;
     }
     return cnt > 2 ? cnt : 2;
 }
 // PktsAcked: the minimum delay and HyStart's exit from slow start (an ACK train as long as the
 // minimum delay, or an RTT rise over it in a round's first eight samples)
-TB_D void on_acked(SndRec &S, int64_t now)
+TB_D void on_acked(Snd &S, int64_t now)
 {
-    if (S.cub_epoch != INT64_MIN && now - S.cub_epoch < EPOCH_GUARD)
+    if (S.rec->cub_epoch != INT64_MIN && now - S.rec->cub_epoch < EPOCH_GUARD)
         return;
     const int64_t rtt = S.srtt;
-    if (S.cub_delaymin == INT64_MIN || S.cub_delaymin > rtt)
-        S.cub_delaymin = rtt;
+    if (S.rec->cub_delaymin == INT64_MIN || S.rec->cub_delaymin > rtt)
+        S.rec->cub_delaymin = rtt;
     const uint32_t w = S.cwnd;
-    if (S.cub_found || w > S.ssthresh || w < 16 * MSS)
+    if (S.rec->cub_found || w > S.ssthresh || w < 16 * MSS)
         return;
-    if (now - S.cub_lastack <= ACK_DELTA)
+    if (now - S.rec->cub_lastack <= ACK_DELTA)
     {
-        S.cub_lastack = now;
-        if (now - S.cub_roundstart > S.cub_delaymin)
-            S.cub_found = 1;
+        S.rec->cub_lastack = now;
+        if (now - S.rec->cub_roundstart > S.rec->cub_delaymin)
+            S.rec->cub_found = 1;
     }
-    if (S.cub_samples >= 8)
+    if (S.rec->cub_samples >= 8)
     {
-        const int64_t dm = S.cub_delaymin;
+        const int64_t dm = S.rec->cub_delaymin;
         const int64_t slack = dm < DELAY_MIN ? DELAY_MIN : dm > DELAY_MAX ? DELAY_MAX : dm;
-        if (S.cub_currrtt > dm + slack)
-            S.cub_found = 1;
+        if (S.rec->cub_currrtt > dm + slack)
+            S.rec->cub_found = 1;
     }
     else
     {
-        if (S.cub_currrtt == INT64_MIN || S.cub_currrtt > rtt)
-            S.cub_currrtt = rtt;
-        S.cub_samples++;
+        if (S.rec->cub_currrtt == INT64_MIN || S.rec->cub_currrtt > rtt)
+            S.rec->cub_currrtt = rtt;
+        S.rec->cub_samples++;
     }
-    if (S.cub_found)
+    if (S.rec->cub_found)
         S.ssthresh = w;
 }
 // IncreaseWindow: slow start by whole segments, else one segment per acks_per_segment ACKs
-TB_D void grow(const Sim &s, SndRec &S, uint32_t segs, uint32_t ack, int64_t now)
+TB_D void grow(const Sim &s, Snd &S, uint32_t segs, uint32_t ack, int64_t now)
 {
     if (!S.cwnd_limited)
         return;
     if (S.cwnd < S.ssthresh)
     {
-        if (ack + 1 > S.cub_endseq)
+        if (ack + 1 > S.rec->cub_endseq)
             new_round(S, now);
         S.cwnd += segs * MSS;
         return;
     }
     if (!segs)
         return;
-    S.cub_cnt += segs;
+    S.rec->cub_cnt += segs;
     const uint32_t cnt = acks_per_segment(s, S, segs, now);
-    if (S.cub_cnt >= cnt)
+    if (S.rec->cub_cnt >= cnt)
     {
         S.cwnd += MSS;
-        S.cub_cnt -= cnt;
+        S.rec->cub_cnt -= cnt;
     }
 }
 // GetSsThresh: beta of the window; the plateau remembered (lowered further when the window did
 // not regain the last one: fast convergence); a new epoch begins at the next increase
-TB_D uint32_t ssthresh(SndRec &S)
+TB_D uint32_t ssthresh(Snd &S)
 {
     const uint32_t w = S.cwnd / MSS;
-    S.cub_lastmax = w < S.cub_lastmax ? x86_u32((w * (1 + BETA)) / 2) : w;
-    S.cub_epoch = INT64_MIN;
+    S.rec->cub_lastmax = w < S.rec->cub_lastmax ? x86_u32((w * (1 + BETA)) / 2) : w;
+    S.rec->cub_epoch = INT64_MIN;
     const uint32_t th = x86_u32(w * BETA);
     return (th > 2 ? th : 2) * MSS;
 }
 // CongestionStateSet(CA_LOSS): the curve and HyStart start over
-TB_D void on_loss(SndRec &S, int64_t now)
+TB_D void on_loss(Snd &S, int64_t now)
 {
-    S.cub_origin = 0;
-    S.cub_k = 0;
-    S.cub_ackcnt = 0;
-    S.cub_tcpcwnd = 0;
-    S.cub_delaymin = INT64_MIN;
-    S.cub_found = 0;
+    S.rec->cub_origin = 0;
+    S.rec->cub_k = 0;
+    S.rec->cub_ackcnt = 0;
+    S.rec->cub_tcpcwnd = 0;
+    S.rec->cub_delaymin = INT64_MIN;
+    S.rec->cub_found = 0;
     new_round(S, now);
 }
 } // namespace cubic
 
 // ------------------------------------------------------------------ NewReno, DCTCP (over Linux Reno)
 // GetSsThresh of the three (reference: src/step.cuh:1055-1063)
-TB_D uint32_t ssthresh_after(HostCtx &c, SndRec &S, uint32_t flight)
+TB_D uint32_t ssthresh_after(HostCtx &c, Snd &S, uint32_t flight)
 {
     if (c.cubic)
         return cubic::ssthresh(S);
@@ -793,7 +818,7 @@ TB_D uint32_t ssthresh_after(HostCtx &c, SndRec &S, uint32_t flight)
 // DCTCP's alpha: once per window of data (up to the byte next after the highest sent when the
 // window began), alpha <- (1 - g) alpha + g F, F the window's ECE-acknowledged fraction, in the fused
 // multiply-add ns-3's -march=native build makes of it
-TB_D void dctcp_acked(SndRec &S, uint32_t segs, uint32_t ack)
+TB_D void dctcp_acked(Snd &S, uint32_t segs, uint32_t ack)
 {
     const uint32_t bytes = segs * MSS;
     S.acked_total += bytes;
@@ -812,7 +837,7 @@ TB_D void dctcp_acked(SndRec &S, uint32_t segs, uint32_t ack)
     S.acked_total = S.acked_ecn = 0;
 }
 // PktsAcked (reference: src/step.cuh:1348-1381)
-TB_D void acked_segments(HostCtx &c, SndRec &S, uint32_t segs, uint32_t ack, int64_t now)
+TB_D void acked_segments(HostCtx &c, Snd &S, uint32_t segs, uint32_t ack, int64_t now)
 {
     if (c.cubic)
         cubic::on_acked(S, now);
@@ -821,7 +846,7 @@ TB_D void acked_segments(HostCtx &c, SndRec &S, uint32_t segs, uint32_t ack, int
 }
 // TcpLinuxReno (DCTCP's window): slow start up to ssthresh; then a segment per window of ACKs,
 // counted in cwnd_cnt
-TB_D void linux_reno_grow(SndRec &S, uint32_t segs)
+TB_D void linux_reno_grow(Snd &S, uint32_t segs)
 {
     if (S.cwnd < S.ssthresh)
     {
@@ -847,7 +872,7 @@ TB_D void linux_reno_grow(SndRec &S, uint32_t segs)
     }
 }
 // TcpNewReno: one segment of slow start per ACK, then MSS^2 / cwnd (at least a byte)
-TB_D void newreno_grow(SndRec &S, uint32_t segs)
+TB_D void newreno_grow(Snd &S, uint32_t segs)
 {
     if (S.cwnd < S.ssthresh && segs)
     {
@@ -861,7 +886,7 @@ TB_D void newreno_grow(SndRec &S, uint32_t segs)
     }
 }
 // IncreaseWindow (reference: src/step.cuh:1383-1440)
-TB_D void grow_window(HostCtx &c, SndRec &S, uint32_t segs, uint32_t ack, int64_t now)
+TB_D void grow_window(HostCtx &c, Snd &S, uint32_t segs, uint32_t ack, int64_t now)
 {
     if (c.cubic)
         cubic::grow(*c.s, S, segs, ack, now);
@@ -872,15 +897,15 @@ TB_D void grow_window(HostCtx &c, SndRec &S, uint32_t segs, uint32_t ack, int64_
 }
 
 // ------------------------------------------------------------------ sending
-TB_D void arm_retx_timer(HostCtx &c, SndRec &S, int64_t now)
+TB_D void arm_retx_timer(HostCtx &c, Snd &S, int64_t now)
 {
     S.rto_at = now + S.rto;
-    chain_child(S.rchain, c.ech, code_lead(S.rto));
+    chain_child(S.rec->rchain, c.ech, code_lead(S.rto));
 }
 // SendDataPacket: a segment of up to max_len bytes at seq (CWR on the first new one after an echo,
 // FIN on the one reaching the end of a closing stream); the retransmission timer starts if idle;
 // the RTT history notes it (reference: src/step.cuh:1129-1172)
-TB_D uint32_t transmit(HostCtx &c, int f, SndRec &S, uint32_t seq, uint32_t max_len, int64_t now)
+TB_D uint32_t transmit(HostCtx &c, int f, Snd &S, uint32_t seq, uint32_t max_len, int64_t now)
 {
     SentList L(*c.s, S);
     bool again = false;
@@ -916,7 +941,7 @@ TB_D uint32_t transmit(HostCtx &c, int f, SndRec &S, uint32_t seq, uint32_t max_
 // SendPendingData: segments while the window has room (a part of a segment only when it ends the
 // data), retransmissions first; nothing more in Open once the FIN is out (reference:
 // src/step.cuh:1175-1199)
-TB_D void send_pending(HostCtx &c, int f, SndRec &S, int64_t now)
+TB_D void send_pending(HostCtx &c, int f, Snd &S, int64_t now)
 {
     if (S.st != S_EST)
         return;
@@ -940,7 +965,7 @@ TB_D void send_pending(HostCtx &c, int f, SndRec &S, int64_t now)
 }
 // DoRetransmit: the first retransmission candidate, else the first unacknowledged byte (reference:
 // src/step.cuh:1202-1212)
-TB_D void retransmit_one(HostCtx &c, int f, SndRec &S, int64_t now)
+TB_D void retransmit_one(HostCtx &c, int f, Snd &S, int64_t now)
 {
     if (S.una >= S.tail)
         return;
@@ -952,7 +977,7 @@ TB_D void retransmit_one(HostCtx &c, int f, SndRec &S, int64_t now)
 }
 // NewAck: the retransmission timer restarts from the estimator (optionally), stops once everything
 // is acknowledged unless a FIN is out; nxt never trails the ACK (reference: src/step.cuh:1445-1464)
-TB_D void new_ack(HostCtx &c, SndRec &S, uint32_t ack, bool restart, int64_t now)
+TB_D void new_ack(HostCtx &c, Snd &S, uint32_t ack, bool restart, int64_t now)
 {
     if (restart)
     {
@@ -967,7 +992,7 @@ TB_D void new_ack(HostCtx &c, SndRec &S, uint32_t ack, bool restart, int64_t now
 // EnterRecovery: a third duplicate (or a lost head) starts fast recovery: the Reno SACK of this
 // duplicate, the head lost, recover = the highest sent, the window to ssthresh and the head resent
 // (reference: src/step.cuh:1467-1481)
-TB_D void enter_recovery(HostCtx &c, int f, SndRec &S, int64_t now)
+TB_D void enter_recovery(HostCtx &c, int f, Snd &S, int64_t now)
 {
     {
         SentList L(*c.s, S);
@@ -983,7 +1008,7 @@ TB_D void enter_recovery(HostCtx &c, int f, SndRec &S, int64_t now)
 }
 // messages whose last byte is acknowledged are complete; the connection is done with the last
 // (and its FIN's ACK, with FIN) (reference: src/step.cuh:1484-1499)
-TB_D void messages_acked(HostCtx &c, SndRec &S, int64_t now)
+TB_D void messages_acked(HostCtx &c, Snd &S, int64_t now)
 {
     MsgRec *M = c.s->msgs + S.m_first;
     for (; S.m_dn < S.m_wr && S.una >= M[S.m_dn].end; S.m_dn++, c.done++)
@@ -999,7 +1024,7 @@ TB_D void messages_acked(HostCtx &c, SndRec &S, int64_t now)
 // a duplicate ACK by congestion state: counted (Recovery counts Reno SACKs instead), Open turns
 // Disorder, and in Disorder the third duplicate (past any earlier recovery point) or a lost head
 // enters recovery; Loss ignores it
-TB_D void duplicate_ack(HostCtx &c, int f, SndRec &S, uint32_t una_before, int64_t now)
+TB_D void duplicate_ack(HostCtx &c, int f, Snd &S, uint32_t una_before, int64_t now)
 {
     switch (S.cong)
     {
@@ -1023,7 +1048,7 @@ TB_D void duplicate_ack(HostCtx &c, int f, SndRec &S, uint32_t una_before, int64
 // an ACK that moves una: `bytes` left the sent list; segments acknowledged with the remainder
 // carried over. Partial ACKs of a recovery retransmit; otherwise the state returns to Open and the
 // window grows (reference: src/step.cuh:1580-1680)
-TB_D void advancing_ack(HostCtx &c, int f, SndRec &S, uint32_t ack, uint32_t una_before, uint32_t bytes, int64_t now)
+TB_D void advancing_ack(HostCtx &c, int f, Snd &S, uint32_t ack, uint32_t una_before, uint32_t bytes, int64_t now)
 {
     uint32_t segs = bytes / MSS;
     S.ack_rem += bytes % MSS;
@@ -1091,7 +1116,7 @@ TB_D void advancing_ack(HostCtx &c, int f, SndRec &S, uint32_t ack, uint32_t una
     new_ack(c, S, ack, true, now);
 }
 // ReceivedAck and ProcessAck, for an ACK with or without ECE (reference: src/step.cuh:1502-1693)
-TB_D void on_ack(HostCtx &c, int f, SndRec &S, uint32_t ack, bool ece, int64_t now)
+TB_D void on_ack(HostCtx &c, int f, Snd &S, uint32_t ack, bool ece, int64_t now)
 {
     if (S.st != S_EST || ack < S.una)
         return;
@@ -1151,7 +1176,7 @@ TB_D void on_ack(HostCtx &c, int f, SndRec &S, uint32_t ack, bool ece, int64_t n
 // the retransmission timeout: everything sent is lost, the timer backs off (at most 60 s), the
 // history is dropped, the window falls to a segment in Loss and sending resumes from the head
 // (reference: src/step.cuh:1695-1725)
-TB_D void on_rto(HostCtx &c, int f, SndRec &S, int64_t now)
+TB_D void on_rto(HostCtx &c, int f, Snd &S, int64_t now)
 {
     S.rto_at = -1;
     if (S.st != S_EST || S.una >= S.tail)
@@ -1177,7 +1202,7 @@ TB_D void on_rto(HostCtx &c, int f, SndRec &S, int64_t now)
 
 // ------------------------------------------------------------------ the receiving socket
 // SYN-ACK, its timer backing off from the connection timeout (reference: src/step.cuh:1729-1743)
-TB_D void send_synack(HostCtx &c, int f, RcvRec &R, int64_t now)
+TB_D void send_synack(HostCtx &c, int f, Rcv &R, int64_t now)
 {
     const int64_t to = CONN_TO_PS << R.syn_n++;
     if (R.synack_t < 0)
@@ -1186,9 +1211,9 @@ TB_D void send_synack(HostCtx &c, int f, RcvRec &R, int64_t now)
     if (R.syn_at >= 0)
         return;
     R.syn_at = now + to;
-    chain_child(R.dchain, c.ech, code_lead(to));
+    chain_child(R.rec->dchain, c.ech, code_lead(to));
 }
-TB_D void rcv_established(RcvRec &R)
+TB_D void rcv_established(Rcv &R)
 {
     if (R.est)
         return;
@@ -1198,7 +1223,7 @@ TB_D void rcv_established(RcvRec &R)
 // DCTCP's receiver: when the CE state flips while an ACK is withheld by the delayed-ACK count, that
 // ACK goes out now with the old state's echo; the state and the sequence it covers are kept
 // (reference: src/step.cuh:1756-1779)
-TB_D void ce_flip(HostCtx &c, int f, RcvRec &R, bool ce, int64_t now)
+TB_D void ce_flip(HostCtx &c, int f, Rcv &R, bool ce, int64_t now)
 {
     if (R.reserved && R.prior_flag && (R.ce_state != 0) != ce)
         rcv_ack(c, f, R, R.prior_rcv_nxt, ce ? ECHO_NEVER : ECHO_FORCE, now);
@@ -1212,7 +1237,7 @@ TB_D void ce_flip(HostCtx &c, int f, RcvRec &R, bool ce, int64_t now)
 }
 // ECN at the receiving socket: a CE mark beyond the last one seen flips the state to CE; any other
 // ECT frame flips it back (reference: src/step.cuh:1785-1800)
-TB_D void rcv_ecn(HostCtx &c, int f, RcvRec &R, const Frame &p, int64_t now)
+TB_D void rcv_ecn(HostCtx &c, int f, Rcv &R, const Frame &p, int64_t now)
 {
     if (!c.dctcp)
         return;
@@ -1226,7 +1251,7 @@ TB_D void rcv_ecn(HostCtx &c, int f, RcvRec &R, const Frame &p, int64_t now)
         ce_flip(c, f, R, false, now);
 }
 // ECN of the ACKs at the sending socket (reference: src/step.cuh:1806-1822)
-TB_D void snd_ecn(HostCtx &c, SndRec &S, const Frame &p)
+TB_D void snd_ecn(HostCtx &c, Snd &S, const Frame &p)
 {
     if (!c.dctcp)
         return;
@@ -1247,7 +1272,7 @@ TB_D void snd_ecn(HostCtx &c, SndRec &S, const Frame &p)
 // disjoint, never touching; a ring at oo_off). The blocks the new bytes overlap or touch fold into
 // one with them; in-order bytes move rcv_nxt to the end of that block, which never enters the ring.
 // False when nothing is new (reference: src/step.cuh:1827-1902)
-TB_D bool rx_add(const Sim &s, RcvRec &R, uint32_t seq, uint32_t end, unsigned &ovf)
+TB_D bool rx_add(const Sim &s, Rcv &R, uint32_t seq, uint32_t end, unsigned &ovf)
 {
     const uint32_t from = seq > R.rcv_nxt ? seq : R.rcv_nxt;
     if (from >= end)
@@ -1336,11 +1361,11 @@ TB_D bool rx_add(const Sim &s, RcvRec &R, uint32_t seq, uint32_t end, unsigned &
         R.rcv_nxt++;
     return true;
 }
-TB_D bool rx_finished(const RcvRec &R) { return R.fin_seq >= 0 && (uint32_t)R.fin_seq < R.rcv_nxt; }
+TB_D bool rx_finished(const RcvCore &R) { return R.fin_seq >= 0 && (uint32_t)R.fin_seq < R.rcv_nxt; }
 
 // the receiver's FIN+ACK; its own retransmission timer from the receiver's estimator (reference:
 // src/step.cuh:1948-1963)
-TB_D void send_fin_ack(HostCtx &c, int f, RcvRec &R, int64_t now)
+TB_D void send_fin_ack(HostCtx &c, int f, Rcv &R, int64_t now)
 {
     R.delack_at = -1;
     R.delack_count = 0;
@@ -1349,31 +1374,31 @@ TB_D void send_fin_ack(HostCtx &c, int f, RcvRec &R, int64_t now)
         return;
     const int64_t to = rto_of(R.srtt, R.rttvar);
     R.frx_at = now + to;
-    chain_child(R.fchain, c.ech, code_lead(to));
+    chain_child(R.rec->fchain, c.ech, code_lead(to));
 }
-TB_D void arm_last_ack(HostCtx &c, RcvRec &R, int64_t now)
+TB_D void arm_last_ack(HostCtx &c, Rcv &R, int64_t now)
 {
     const int64_t to = rto_raw(R.srtt, R.rttvar); // (LastAckTimeout takes the RTO unclamped)
     R.last_at = now + to;
-    chain_child(R.dchain, c.ech, code_lead(to));
+    chain_child(R.rec->dchain, c.ech, code_lead(to));
 }
 // DoPeerClose and the application's Close right after: FIN+ACK, LAST_ACK (reference:
 // src/step.cuh:1974-1984)
-TB_D void do_peer_close(HostCtx &c, int f, RcvRec &R, int64_t now)
+TB_D void do_peer_close(HostCtx &c, int f, Rcv &R, int64_t now)
 {
     R.st = R_LAST_ACK;
     send_fin_ack(c, f, R, now);
     R.last_n = DATA_RETRIES;
     arm_last_ack(c, R, now);
 }
-TB_D void rcv_closed(RcvRec &R)
+TB_D void rcv_closed(Rcv &R)
 {
     R.st = R_CLOSED;
     R.last_at = R.frx_at = R.delack_at = -1;
 }
 // ReceivedData: new bytes into the buffer; an ACK at once for a gap (or a filled one) or every
 // second segment, else the delayed-ACK timer (reference: src/step.cuh:1994-2036)
-TB_D void received_data(HostCtx &c, int f, RcvRec &R, uint32_t seq, uint32_t len, bool fin, int64_t now)
+TB_D void received_data(HostCtx &c, int f, Rcv &R, uint32_t seq, uint32_t len, bool fin, int64_t now)
 {
     const uint32_t expected = R.rcv_nxt;
     if (!rx_add(*c.s, R, seq, seq + len, c.ovf))
@@ -1397,11 +1422,11 @@ TB_D void received_data(HostCtx &c, int f, RcvRec &R, uint32_t seq, uint32_t len
     if (R.delack_at >= 0)
         return;
     R.delack_at = now + DELACK_PS;
-    chain_child(R.dchain, c.ech, code_lead(DELACK_PS));
+    chain_child(R.rec->dchain, c.ech, code_lead(DELACK_PS));
 }
 // a data segment or FIN at the receiving socket: old data get a duplicate ACK without ECE; a FIN
 // is taken in order only; LAST_ACK closes on the FIN's ACK (reference: src/step.cuh:2040-2101)
-TB_D void on_data(HostCtx &c, int f, RcvRec &R, const Frame &p, int64_t now)
+TB_D void on_data(HostCtx &c, int f, Rcv &R, const Frame &p, int64_t now)
 {
     if (!R.up || R.st == R_CLOSED)
         return;
@@ -1446,7 +1471,7 @@ TB_D void on_data(HostCtx &c, int f, RcvRec &R, const Frame &p, int64_t now)
 // ------------------------------------------------------------------ the application
 // FlowSender::Write: the messages due join the stream (the last one closes it, with FIN); the send
 // is deferred a step as Socket::Send defers SendPendingData (reference: src/step.cuh:2118-2144)
-TB_D void app_write(HostCtx &c, int f, SndRec &S, int64_t now)
+TB_D void app_write(HostCtx &c, int f, Snd &S, int64_t now)
 {
     if (S.m_wr >= S.m_due)
         return;
@@ -1461,7 +1486,7 @@ TB_D void app_write(HostCtx &c, int f, SndRec &S, int64_t now)
     if (S.cwnd <= inflight(S) || S.syn_at >= 0)
         return;
     S.syn_at = now + 1;
-    chain_child(S.schain, c.ech, CODE_STEP);
+    chain_child(S.rec->schain, c.ech, CODE_STEP);
     timer_in_slot(c, now + 1, f, 2);
 }
 TB_D bool add_active(const Sim &s, int *list, int &n, int f, unsigned &ovf)
@@ -1480,13 +1505,14 @@ TB_D void app_event(HostCtx &c, HostRec &hr, int *act_snd, int m, int64_t now)
 {
     const WorldDesc &wd = *c.wd;
     const int f = c.s->msgs[m].conn;
-    SndRec &S = c.s->snd[f];
+    Snd S(c.s->snd[f]);
     if (S.m_first != m)
     {
         chain_msg_root(c.ech, m - wd.msg0);
         S.m_due++;
         if (S.st == S_EST)
             app_write(c, f, S, now);
+        S.store();
         return;
     }
     chain_app_root(c.ech, hr.local, f - wd.conn0);
@@ -1497,44 +1523,40 @@ TB_D void app_event(HostCtx &c, HostRec &hr, int *act_snd, int m, int64_t now)
         cubic::new_round(S, now);
     S.rto = CONN_TO_PS;
     S.syn_at = now + CONN_TO_PS;
-    chain_child(S.rchain, c.ech, code_lead(CONN_TO_PS));
+    chain_child(S.rec->rchain, c.ech, code_lead(CONN_TO_PS));
     S.timing_time = now;
     emit_snd(c, f, S, F_SYN, 0, SYN_LEN, now);
+    S.store();
 }
 
 // ------------------------------------------------------------------ timers and frames
 // a timer of the slot fires if it is still the one armed (reference: src/step.cuh:2380-2440)
-TB_D void timer_event(HostCtx &c, const Due &d, int64_t now)
+TB_D void snd_timer(HostCtx &c, int f, Snd &S, const Due &d, int64_t now)
 {
-    const Sim &s = *c.s;
-    const int f = d.flow;
-    if (d.kind == 0 || d.kind == 2)
+    if (d.kind == 0)
     {
-        SndRec &S = s.snd[f];
-        if (d.kind == 0)
-        {
-            if (S.rto_at == d.at)
-                on_rto(c, f, S, now);
-            return;
-        }
-        if (S.syn_at != d.at)
-            return;
-        if (S.st == S_EST)
-        {
-            S.syn_at = -1; // the deferred SendPendingData
-            send_pending(c, f, S, now);
-        }
-        else if (S.st == S_SYN_SENT)
-        {
-            // the SYN again, the connection timeout doubled
-            S.rto = CONN_TO_PS << ++S.syn_tries;
-            S.syn_at = now + S.rto;
-            chain_child(S.rchain, c.ech, code_lead(S.rto));
-            emit_snd(c, f, S, F_SYN, 0, SYN_LEN, now);
-        }
+        if (S.rto_at == d.at)
+            on_rto(c, f, S, now);
         return;
     }
-    RcvRec &R = s.rcv[f];
+    if (S.syn_at != d.at)
+        return;
+    if (S.st == S_EST)
+    {
+        S.syn_at = -1; // the deferred SendPendingData
+        send_pending(c, f, S, now);
+    }
+    else if (S.st == S_SYN_SENT)
+    {
+        // the SYN again, the connection timeout doubled
+        S.rto = CONN_TO_PS << ++S.syn_tries;
+        S.syn_at = now + S.rto;
+        chain_child(S.rec->rchain, c.ech, code_lead(S.rto));
+        emit_snd(c, f, S, F_SYN, 0, SYN_LEN, now);
+    }
+}
+TB_D void rcv_timer(HostCtx &c, int f, Rcv &R, const Due &d, int64_t now)
+{
     switch (d.kind)
     {
     case 1: // delayed ACK
@@ -1569,41 +1591,50 @@ TB_D void timer_event(HostCtx &c, const Due &d, int64_t now)
         send_fin_ack(c, f, R, now);
     }
 }
+TB_D void timer_event(HostCtx &c, const Due &d, int64_t now)
+{
+    if (d.kind == 0 || d.kind == 2)
+    {
+        Snd S(c.s->snd[d.flow]);
+        snd_timer(c, d.flow, S, d, now);
+        S.store();
+        return;
+    }
+    Rcv R(c.s->rcv[d.flow]);
+    rcv_timer(c, d.flow, R, d, now);
+    R.store();
+}
 
 // a frame at its destination host: at the sender a SYN-ACK (connected: ACK, then the application's
 // write), an ACK, or the receiver's FIN+ACK (TIME_WAIT after its ACK); at the receiver a SYN (the
 // SYN-ACK, the fork's ScheduleNow), data or FIN, or the handshake's ACK (reference: src/step.cuh:2147-2236)
-TB_D void on_frame(HostCtx &c, HostRec &hr, const Frame &p, int64_t now)
+TB_D void snd_frame(HostCtx &c, int f, Snd &S, const Frame &p, int64_t now)
 {
-    const Sim &s = *c.s;
-    const int f = (int)p.flow;
-    if (p.to_sender)
+    if (p.flags & F_SYN)
     {
-        SndRec &S = s.snd[f];
-        if (p.flags & F_SYN)
-        {
-            if (S.st != S_SYN_SENT)
-                return;
-            S.st = S_EST;
-            S.syn_at = -1;
-            rtt_update(S, now - S.timing_time);
-            emit_snd(c, f, S, F_ACK, 0, CTRL_LEN, now);
-            chain_child(c.ech, c.ech, CODE_NOW); // (ConnectionSucceeded is ScheduleNow'd)
-            app_write(c, f, S, now);
+        if (S.st != S_SYN_SENT)
             return;
-        }
-        if (S.fin & FIN_TW)
-            return;
-        snd_ecn(c, S, p);
-        on_ack(c, f, S, p.sa, p.flags & F_ECE, now);
-        if (p.flags & F_FIN)
-        {
-            S.fin |= FIN_TW;
-            emit_snd(c, f, S, F_ACK, 1, CTRL_LEN, now);
-        }
+        S.st = S_EST;
+        S.syn_at = -1;
+        rtt_update(S, now - S.timing_time);
+        emit_snd(c, f, S, F_ACK, 0, CTRL_LEN, now);
+        chain_child(c.ech, c.ech, CODE_NOW); // (ConnectionSucceeded is ScheduleNow'd)
+        app_write(c, f, S, now);
         return;
     }
-    RcvRec &R = s.rcv[f];
+    if (S.fin & FIN_TW)
+        return;
+    snd_ecn(c, S, p);
+    on_ack(c, f, S, p.sa, p.flags & F_ECE, now);
+    if (p.flags & F_FIN)
+    {
+        S.fin |= FIN_TW;
+        emit_snd(c, f, S, F_ACK, 1, CTRL_LEN, now);
+    }
+}
+TB_D void rcv_frame(HostCtx &c, HostRec &hr, int f, Rcv &R, const Frame &p, int64_t now)
+{
+    const Sim &s = *c.s;
     if (p.flags & F_SYN)
     {
         if (!R.up)
@@ -1634,6 +1665,20 @@ TB_D void on_frame(HostCtx &c, HostRec &hr, const Frame &p, int64_t now)
         if (R.st == R_LAST_ACK)
             rcv_closed(R);
     }
+}
+TB_D void on_frame(HostCtx &c, HostRec &hr, const Frame &p, int64_t now)
+{
+    const int f = (int)p.flow;
+    if (p.to_sender)
+    {
+        Snd S(c.s->snd[f]);
+        snd_frame(c, f, S, p, now);
+        S.store();
+        return;
+    }
+    Rcv R(c.s->rcv[f]);
+    rcv_frame(c, hr, f, R, p, now);
+    R.store();
 }
 
 } // namespace tb
