@@ -73,8 +73,8 @@ TB_HD uint16_t code_tc(int len) { return (uint16_t)len; }
 TB_HD uint16_t code_arrival(int len) { return (uint16_t)(2048 + len); }
 TB_HD uint16_t code_lead(int64_t lead_ps)
 {
-    int64_t c = 4096 + lead_ps / 16000;
-    return (uint16_t)(c < 0xFFFE ? c : 0xFFFE);
+    // (saturated from 61438 units on, as every retransmission timeout's is: the quotient of a 32-bit value)
+    return lead_ps < 61438ll * 16000 ? (uint16_t)(4096 + (uint32_t)lead_ps / 16000) : (uint16_t)0xFFFE;
 }
 
 TB_HD void chain_clear(Chain &c)

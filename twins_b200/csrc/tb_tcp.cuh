@@ -44,18 +44,25 @@ struct Snd : SndCore
 {
     SndRec *rec;
     TB_D explicit Snd(SndRec &r) : SndCore(r), rec(&r) {}
-    TB_D void store() const { store_core(rec, this, sizeof(SndCore)); }
-    // the words of a core that change, back to its record
-    TB_D static void store_core(void *to, const void *from, size_t bytes)
+    TB_D void store() const { store_core<SndCore>(rec, this); }
+    // the words of a core that change, back to its record (16 bytes at a time, said in so many
+    // words: a memcpy to a pointer of unknown alignment stored byte by byte, 1,300 cycles of an
+    // ACK's 8,500)
+    template <class Core>
+    TB_D static void store_core(Core *to, const Core *from)
     {
-        memcpy((char *)to + REC_FIXED, (const char *)from + REC_FIXED, bytes - REC_FIXED);
+        const uint4 *a = reinterpret_cast<const uint4 *>(from);
+        uint4 *b = reinterpret_cast<uint4 *>(to);
+#pragma unroll
+        for (int i = REC_FIXED / 16; i < (int)(sizeof(Core) / 16); i++)
+            b[i] = a[i];
     }
 };
 struct Rcv : RcvCore
 {
     RcvRec *rec;
     TB_D explicit Rcv(RcvRec &r) : RcvCore(r), rec(&r) {}
-    TB_D void store() const { Snd::store_core(rec, this, sizeof(RcvCore)); }
+    TB_D void store() const { Snd::store_core<RcvCore>(rec, this); }
 };
 static_assert(offsetof(SndCore, m_due) == REC_FIXED && offsetof(RcvCore, fin_on) == REC_FIXED && sizeof(SndCore) % 16 == 0 && sizeof(RcvCore) % 16 == 0,
               "cores move as 16-byte words");
@@ -881,8 +888,10 @@ TB_D void newreno_grow(Snd &S, uint32_t segs)
     }
     if (S.cwnd >= S.ssthresh && segs)
     {
-        const double step = (double)MSS * MSS / S.cwnd;
-        S.cwnd += (uint32_t)(step > 1.0 ? step : 1.0);
+        // (ns-3 truncates the double quotient: an inexact one lies at least 2^-22 of its size from a
+        // whole number, far beyond a double's rounding, so the integer quotient is the same)
+        const uint32_t step = MSS * MSS / S.cwnd;
+        S.cwnd += step > 1 ? step : 1;
     }
 }
 // IncreaseWindow (reference: src/step.cuh:1383-1440)
