@@ -57,7 +57,21 @@ __device__ __forceinline__ unsigned ld_gen(const unsigned *p)
     return v;
 }
 
-__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+// An L1 line brought in ahead by a load whose value nobody waits for (prefetch.global.L1 left the
+// loads that follow it as slow as without it here: with the loads, and every sector and ring head an
+// event reads among them, k=16 takes 89.9 ms against 94.1 ms, three k=8 worlds 237 against 244 ms).
+__device__ __forceinline__ void prefetch_l1(const void *p)
+{
+    unsigned v;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    (void)v;
+}
+// (the L1 fills by 32-byte sectors: a prefetch per sector, not per line)
+__device__ __forceinline__ void prefetch_l1(const void *p, int bytes)
+{
+    for (int b = 0; b < bytes; b += 32)
+        prefetch_l1((const char *)p + b);
+}
 
 // the stream's look-ahead rows (tb_common.cuh), in global memory, read through the read-only path
 __device__ const RngAhead g_rng_ahead = make_rng_ahead();
@@ -270,6 +284,7 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
             for (int i = lane; i < n; i += 32)
                 frame_load_link(sh.fr()[i], i < n2 ? msg_frames(s, t - 2, link) + i : msg_frames(s, t - 1, link) + (i - n2));
         __syncwarp();
+        const bool cubic = s.worlds[w].cc == CC_CUBIC;
         if (staged)
             for (int i = lane; i < n; i += 32)
             {
@@ -277,21 +292,25 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
                 if (f.to_sender)
                 {
                     const SndRec *S = &s.snd[f.flow];
-                    for (int b = 0; b < (int)sizeof(SndRec); b += 128)
-                        prefetch_l1((const char *)S + b);
+                    prefetch_l1(S, sizeof(SndCore));
+                    prefetch_l1(&S->rchain, sizeof(Chain));
+                    if (cubic)
+                        prefetch_l1((const char *)S + sizeof(SndCore), 80);
+                    // the heads of its sent list and RTT history, where the list grows, its message
                     const uint64_t off = S->it_off;
-                    prefetch_l1(&s.it_start[off + S->it_head]);
-                    prefetch_l1(&s.it_fl[off + 4 * (S->it_head >> 3)]); // (the flag word of the head's eight)
-                    const uint32_t hh = S->h_head;
-                    prefetch_l1(&s.h_seq[off + hh]);
-                    prefetch_l1(&s.h_end[off + hh]);
-                    prefetch_l1(&s.h_t[off + hh]);
+                    const uint32_t cap = S->it_cap, hd = S->it_head, hh = S->h_head, n = S->it_n;
+                    const uint32_t tl = hd + n < cap ? hd + n : hd + n - cap;
+                    prefetch_l1(&s.it_start[off + hd], min(64, (int)(4 * (cap - hd))));
+                    prefetch_l1(&s.it_fl[off + 4 * (hd >> 3)]); // (the flag word of the head's eight)
+                    prefetch_l1(&s.it_fl[off + 4 * (tl >> 3)]);
+                    prefetch_l1(&s.h_end[off + hh], min(64, (int)(4 * (cap - hh))));
+                    prefetch_l1(&s.h_t[off + hh], min(96, (int)(8 * (cap - hh))));
+                    if (S->m_dn < S->m_cnt)
+                        prefetch_l1(&s.msgs[S->m_first + S->m_dn].end);
                 }
                 else
                 {
-                    const RcvRec *R = &s.rcv[f.flow];
-                    for (int b = 0; b < (int)sizeof(RcvRec); b += 128)
-                        prefetch_l1((const char *)R + b);
+                    prefetch_l1(&s.rcv[f.flow], sizeof(RcvRec));
                 }
             }
         if (lane < 8 && lane < hr.q_size)
@@ -299,7 +318,7 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
             int at = hr.q_head + lane;
             if (at >= s.ring)
                 at -= s.ring;
-            prefetch_l1(&s.host_ring[(size_t)h * s.ring + at]);
+            prefetch_l1(&s.host_ring[(size_t)h * s.ring + at], sizeof(Frame));
         }
         if (sh.due_fit(DUE_CAP * sizeof(Due)))
         {
@@ -471,7 +490,7 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
         {
             const Frame *ring = s.port_ring + (size_t)(sr.port0 + lane) * s.ring;
             for (int j = 0; j < 9 && j < qn; j++)
-                prefetch_l1(&ring[qh + j < s.ring ? qh + j : qh + j - s.ring]);
+                prefetch_l1(&ring[qh + j < s.ring ? qh + j : qh + j - s.ring], sizeof(Frame));
         }
         __syncwarp();
         // the frames: copied, their place in the window
