@@ -48,10 +48,10 @@ TB_D bool rcv_idle_for_good(const RcvRec &R)
 // prune_later: the active lists are left unpruned and *wake counts only the host's queue and its
 // next application start; the caller prunes them (prune_lists_warp) and lowers the wake-up to the
 // earliest timer of the connections that stay. `due`: the timers due in the slot, already collected
-// in this function's scan order (the first DUE_CAP of them; due_ovf more were left out), or null
-// to scan the active lists here.
+// in this function's scan order (the first DUE_CAP of them; due_ovf more were left out), with room
+// for DUE_CAP, or null to scan the active lists here.
 TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, unsigned *ties_out, unsigned *done_out,
-                    const Frame *stage = nullptr, int n2 = -1, int n1 = -1, bool prune_later = false, const Due *due = nullptr,
+                    const Frame *stage = nullptr, int n2 = -1, int n1 = -1, bool prune_later = false, Due *due = nullptr,
                     int due_n = 0, int due_ovf = 0)
 {
     const int64_t S0 = t * SLOT_PS, E0 = S0 + SLOT_PS;
@@ -112,10 +112,10 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
     const int ns = hr.n_snd, nr = hr.n_rcv;
     c.nd = 0;
     c.di = 0;
+    Due own[DUE_CAP];
+    c.due = due ? due : own;
     if (due)
     {
-        for (int i = 0; i < due_n; i++)
-            c.due[i] = due[i];
         c.nd = due_n;
         c.ovf += due_ovf;
     }

@@ -30,7 +30,7 @@ struct HostCtx
     bool dctcp, cubic;
     Egress nic;
     Chain ech;
-    Due due[DUE_CAP];
+    Due *due; // [DUE_CAP], beside the context: an array indexed at run time would keep all of it in memory
     int nd, di;
     int64_t slot_end;
     unsigned retx, rtos, ovf, done;
@@ -43,8 +43,18 @@ struct HostCtx
 struct Snd : SndCore
 {
     SndRec *rec;
-    TB_D explicit Snd(SndRec &r) : SndCore(r), rec(&r) {}
+    TB_D explicit Snd(SndRec &r) : rec(&r) { load_core<SndCore>(this, &r); }
     TB_D void store() const { store_core<SndCore>(rec, this); }
+    // a core from its record
+    template <class Core>
+    TB_D static void load_core(Core *to, const Core *from)
+    {
+        const uint4 *a = reinterpret_cast<const uint4 *>(from);
+        uint4 *b = reinterpret_cast<uint4 *>(to);
+#pragma unroll
+        for (int i = 0; i < (int)(sizeof(Core) / 16); i++)
+            b[i] = a[i];
+    }
     // the words of a core that change, back to its record (16 bytes at a time, said in so many
     // words: a memcpy to a pointer of unknown alignment stored byte by byte, 1,300 cycles of an
     // ACK's 8,500)
@@ -61,7 +71,7 @@ struct Snd : SndCore
 struct Rcv : RcvCore
 {
     RcvRec *rec;
-    TB_D explicit Rcv(RcvRec &r) : RcvCore(r), rec(&r) {}
+    TB_D explicit Rcv(RcvRec &r) : rec(&r) { Snd::load_core<RcvCore>(this, &r); }
     TB_D void store() const { Snd::store_core<RcvCore>(rec, this); }
 };
 static_assert(offsetof(SndCore, m_due) == REC_FIXED && offsetof(RcvCore, fin_on) == REC_FIXED && sizeof(SndCore) % 16 == 0 && sizeof(RcvCore) % 16 == 0,
