@@ -670,6 +670,8 @@ void build_image(const HostWorld &w, const Place &pl, WorldImage &img)
         S_.dst_local = R.dst_local = first.dst;
         S_.hash_data = w.hash_data[cc];
         S_.hash_ack = R.hash_ack = w.hash_ack[cc];
+        S_.up = S_.hash_data % (uint32_t)w.ecmp_n;
+        R.up_ack = R.hash_ack % (uint32_t)w.ecmp_n;
         S_.m_first = pl.msg0 + w.row_msg[cr[0]];
         S_.m_cnt = (int)cr.size();
         S_.fin_on = R.fin_on = (uint8_t)(w.p.fin != 0);

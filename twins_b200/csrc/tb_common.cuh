@@ -12,10 +12,12 @@
 #define TB_HD __host__ __device__ __forceinline__
 #define TB_HDI __host__ __device__ inline
 #define TB_D __device__ __forceinline__
+#define TB_DN __device__ __noinline__
 #else
 #define TB_HD inline
 #define TB_HDI inline
 #define TB_D inline
+#define TB_DN inline
 #endif
 
 namespace tb

@@ -124,7 +124,9 @@ TB_D void qtrace_enqueue(const Sim &s, int node, int dev, const Frame &g, int ba
 // not started, each stamped with its enqueue time; the wire is busy until `busy_until` with the
 // frame that began at `began`, whose chain is *tx_chain. A frame begins at max(its enqueue time,
 // busy_until); its transmission's copy, stamped with its arrival at the far end, goes to this
-// slot's link message `msg` (at most MAX_TX; more is counted as an overflow).
+// slot's link message `msg` (at most MAX_TX; more is counted as an overflow). (Hosts that share a warp,
+// and a switch port in a slot beyond the staging area; HostNic and sw_egress_staged are the same device a
+// slot at a time.)
 struct Egress
 {
     Frame *ring;
@@ -246,4 +248,175 @@ struct Egress
         return true;
     }
 };
+// The sending end of a host that has a warp of its own (the same device). The sockets never look at it, so the slot's events only
+// append the frames they offer, each stamped with its time, to a list on chip, and `run` plays the
+// list through the device, a frame per iteration that starts on the wire or joins the queue, in
+// offsets in the slot; what is still queued then joins the ring. (With the device's code at every
+// place that sends a frame, and each frame written to the ring in memory and read back to start,
+// the event loop took more instructions and waited on every frame: a load from a line that was just
+// stored takes 600 cycles longer than another.) OFFER_KICK in a
+// frame's to_sender: offered by a ScheduleNow'd event of its instant.
+constexpr uint8_t OFFER_KICK = 2;
+constexpr int OUT_FRAMES = 16; // the list's capacity (a slot takes 8 full frames; more frames in a slot are played in parts)
+struct HostNic
+{
+    const Sim *s;
+    Frame *ring;
+    int cap, head, size; // the ring
+    int busy, began, tx_len; // the wire: busy until `busy` with a frame of tx_len bytes that began at `began` (offsets)
+    int idle_at;         // the last start this slot on an idle wire (-1: none)
+    int red_k, qcap;
+    int64_t S0;
+    Frame *msg;
+    Chain *wire;         // the chain of the frame on the wire
+    int n_out;
+    unsigned drops, marks, ovf, offered;
+    int node;
+
+    TB_D void open(const Sim &s_, HostRec &hr, Frame *ring_, const WorldDesc &wd, int64_t S0_, Frame *msg_)
+    {
+        s = &s_;
+        ring = ring_;
+        cap = s_.ring;
+        head = hr.q_head;
+        size = hr.q_size;
+        S0 = S0_;
+        busy = -1;
+        began = -(int)SLOT_PS;
+        tx_len = 0;
+        if (hr.link_free >= S0)
+        {
+            busy = (int)(hr.link_free - S0);
+            tx_len = (int)((uint32_t)(hr.link_free - hr.last_start) / (uint32_t)PS_PER_BYTE);
+            began = busy - tx_len * (int)PS_PER_BYTE;
+        }
+        idle_at = -1;
+        red_k = wd.red_k;
+        qcap = wd.qcap;
+        msg = msg_;
+        wire = &hr.last;
+        n_out = 0;
+        drops = marks = ovf = offered = 0;
+        node = hr.local;
+    }
+    TB_D void close(HostRec &hr) const
+    {
+        hr.q_head = head;
+        hr.q_size = size;
+        if (n_out)
+        {
+            hr.link_free = S0 + busy;
+            hr.last_start = S0 + began;
+        }
+    }
+
+    // the frames list[0..n), offered in this order, and every start by `until` (an offset). A queued
+    // frame begins when the wire gets free (it was queued because the wire was busy beyond its
+    // offer), behind the frame on the wire, whose chain is its parent's; one offered at an idle wire
+    // begins at once, its chain unchanged. RED as in Egress; a ScheduleNow'd event also sees the
+    // Wake of a start on an idle wire at its own instant.
+    TB_D void run_list(Frame *list, int n, int until)
+    {
+        constexpr int SLOT = (int)SLOT_PS;
+        Chain on = *wire;
+        int i = 0, jq = 0, lq = 0; // the next offer; list[jq]: the first queued from the list; their number
+        const int n_out0 = n_out;
+        for (;;)
+        {
+            const int waiting = size + lq;
+            const int ta = i < n ? (int)(list[i].ts - S0) : until;
+            const bool room = n_out < MAX_TX, start = waiting > 0 && busy < SLOT && busy <= ta && room;
+            if (!start && i >= n)
+                break;
+            Frame f;
+            frame_copy(&f, start ? (size ? &ring[head] : &list[jq]) : &list[i]);
+            if (!start)
+                offered++;
+            const bool idle = waiting == 0 && busy <= ta && room;
+            if (start || idle)
+            {
+                const bool behind = start || (busy == ta && tx_len > 0);
+                if (behind)
+                    chain_child(f.ch, on, code_tc(tx_len));
+                else
+                    idle_at = ta;
+#ifdef TB_QTRACE
+                if (!start)
+                    qtrace_enqueue(*s, node, 1, f, 0, f.ts);
+#endif
+                on = f.ch;
+                began = start ? busy : ta;
+                tx_len = f.len;
+                busy = began + tx_len * (int)PS_PER_BYTE;
+                f.ts = S0 + busy + PROP_PS;
+                f.to_sender &= 1;
+                frame_store_link(&msg[n_out++], f);
+                if (!start)
+                {
+                    i++;
+                    jq = i;
+                }
+                else if (size)
+                {
+                    head = head + 1 == cap ? 0 : head + 1;
+                    size--;
+                }
+                else
+                {
+                    lq--;
+                    jq++;
+                    while (jq < i && list[jq].len == 0)
+                        jq++; // (dropped)
+                }
+                continue;
+            }
+            // an offer that finds the wire busy, or frames waiting
+            const bool woken = began < ta || ((f.to_sender & OFFER_KICK) && idle_at == ta);
+            const int backlog = !waiting || busy <= ta ? waiting : waiting - (woken ? 1 : 0);
+            bool gone = false;
+            ovf += !room;
+            if (backlog >= red_k && backlog > 1)
+            {
+                if (f.flags & F_ECT)
+                {
+                    f.flags |= F_CE;
+                    list[i].flags = f.flags;
+                    marks++;
+                }
+                else
+                    gone = true;
+            }
+            gone |= backlog >= qcap;
+            drops += gone;
+#ifdef TB_QTRACE
+            if (!gone)
+                qtrace_enqueue(*s, node, 1, f, backlog, f.ts);
+#endif
+            if (!gone && waiting == cap)
+            {
+                ovf++;
+                gone = true;
+            }
+            if (gone)
+                list[i].len = 0;
+            if (lq == 0)
+                jq = gone ? i + 1 : i;
+            lq += !gone;
+            i++;
+        }
+        for (; lq; jq++)
+        {
+            if (list[jq].len == 0)
+                continue;
+            const int at = head + size;
+            list[jq].to_sender &= 1;
+            frame_copy(&ring[at < cap ? at : at - cap], &list[jq]);
+            size++;
+            lq--;
+        }
+        if (n_out != n_out0)
+            *wire = on;
+    }
+};
+
 } // namespace tb

@@ -372,7 +372,7 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
     bool act = false;
     if (run)
     {
-        act = host_step(s, h, t - t0, t, &wake, &ties, &done, stage, n2, n1, !MANY, due, due_n, due_ovf);
+        act = host_step<!MANY>(s, h, t - t0, t, &wake, &ties, &done, sh.offered(), stage, n2, n1, due, due_n, due_ovf);
         if constexpr (MANY)
             host_report(s, w, t0, act, wake, done);
     }

@@ -45,13 +45,16 @@ TB_D bool rcv_idle_for_good(const RcvRec &R)
 // `stage`: the host's link messages of slots gt-2 and gt-1 copied to shared memory by its warp
 // (msg[gt-2] then msg[gt-1], n2 and n1 frames as their tags count), or null to read them in place
 // (n2, n1 < 0: read the tags).
-// prune_later: the active lists are left unpruned and *wake counts only the host's queue and its
-// next application start; the caller prunes them (prune_lists_warp) and lowers the wake-up to the
-// earliest timer of the connections that stay. `due`: the timers due in the slot, already collected
+// KEEP (one host per warp): the records last used stay in registers between events (Recs); the active
+// lists are left unpruned and *wake counts only the host's queue and its next application start; the
+// caller prunes them (prune_lists_warp) and lowers the wake-up to the earliest timer of the
+// connections that stay. `due`: the timers due in the slot, already collected
 // in this function's scan order (the first DUE_CAP of them; due_ovf more were left out), with room
 // for DUE_CAP, or null to scan the active lists here.
-TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, unsigned *ties_out, unsigned *done_out,
-                    const Frame *stage = nullptr, int n2 = -1, int n1 = -1, bool prune_later = false, Due *due = nullptr,
+// `out` (KEEP): the list of the frames its events offer, room for OUT_FRAMES.
+template <bool KEEP>
+TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, unsigned *ties_out, unsigned *done_out, Frame *out,
+                    const Frame *stage = nullptr, int n2 = -1, int n1 = -1, Due *due = nullptr,
                     int due_n = 0, int due_ovf = 0)
 {
     const int64_t S0 = t * SLOT_PS, E0 = S0 + SLOT_PS;
@@ -95,15 +98,26 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
     c.slot_end = E0;
     c.retx = c.rtos = c.ovf = c.done = 0;
     c.pkts = c.snd_pkts = 0;
-    Egress &nic = c.nic;
-    nic.open(s.host_ring + (size_t)h * s.ring, s.ring, hr.q_head, hr.q_size, hr.link_free, hr.last_start, &hr.last, wd.red_k, wd.qcap, E0,
-             s.msg + msg_index(s, gt, h) * MAX_TX);
+    HostNic nic;
+    c.list = KEEP;
+    c.nic = &nic;
+    c.out = out;
+    c.out_n = 0;
+    c.kicked = -1;
+    if (KEEP)
+        nic.open(s, hr, s.host_ring + (size_t)h * s.ring, wd, S0, s.msg + msg_index(s, gt, h) * MAX_TX);
+    else
+    {
+        c.eg.open(s.host_ring + (size_t)h * s.ring, s.ring, hr.q_head, hr.q_size, hr.link_free, hr.last_start, &hr.last, wd.red_k, wd.qcap,
+                  E0, s.msg + msg_index(s, gt, h) * MAX_TX);
 #ifdef TB_QTRACE
-    nic.qs = &s;
-    nic.qnode = hr.local;
-    nic.qdev = 1;
+        c.eg.qs = &s;
+        c.eg.qnode = hr.local;
+        c.eg.qdev = 1;
 #endif
+    }
     unsigned ties = 0;
+    Recs<KEEP> recs;
 
     TB_PHASE(0)
     // timers due in this slot (new timers lie >= 10 us ahead, except the 1 ps Send deferral,
@@ -207,17 +221,19 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
         if (now < S0)
             now = S0;
         TB_PHASE(2)
-        nic.advance(now);
-        TB_PHASE(8)
+        if (!KEEP)
+            c.eg.advance(now);
         if (now == tp)
         {
-            app_event(c, hr, act_snd, pm, now);
+            app_event(c, recs, hr, act_snd, pm, now);
             pn++;
             next_pend();
             TB_PHASE(10)
             continue;
         }
         bool timer = now == td;
+        if (KEEP && timer && recs.S.f == c.due[c.di].flow)
+            recs.flush(); // (its chain is read from the record)
         if (timer && now == tr)
         {
             // a timer and an arrival at the same instant: the one scheduled first
@@ -232,7 +248,7 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
         {
             const Due d = c.due[c.di++];
             c.ech = due_chain(s, d);
-            timer_event(c, d, now);
+            timer_event(c, recs, d, now);
             TB_PHASE(10)
             continue;
         }
@@ -245,22 +261,39 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
         c.pkts++;
         c.snd_pkts += p.to_sender;
         chain_child(c.ech, p.ch, code_arrival(p.len));
-        on_frame(c, hr, p, now);
+        on_frame(c, recs, hr, p, now);
         TB_PHASE(9)
     }
+    if (KEEP)
+        recs.flush();
     TB_PHASE(2)
-    nic.advance(E0 - 1);
-    tag_store(&s.msg_tag[msg_index(s, gt, h)], (int64_t)gt << 16 | nic.n_out);
-    hr.q_head = nic.head;
-    hr.q_size = nic.size;
-    hr.link_free = nic.busy_until;
-    hr.last_start = nic.began;
+    int sent, held;
+    unsigned drops, marks, ovf, offered;
+    if (KEEP)
+    {
+        nic_run(&nic, c.out, c.out_n, (int)SLOT_PS - 1);
+        nic.close(hr);
+        sent = nic.n_out, held = nic.size;
+        drops = nic.drops, marks = nic.marks, ovf = nic.ovf, offered = nic.offered;
+    }
+    else
+    {
+        c.eg.advance(E0 - 1);
+        hr.q_head = c.eg.head;
+        hr.q_size = c.eg.size;
+        hr.link_free = c.eg.busy_until;
+        hr.last_start = c.eg.began;
+        sent = c.eg.n_out, held = c.eg.size;
+        drops = c.eg.drops, marks = c.eg.marks, ovf = c.eg.ovf, offered = c.eg.offered;
+    }
+    TB_PHASE(8)
+    tag_store(&s.msg_tag[msg_index(s, gt, h)], (int64_t)gt << 16 | sent);
     hr.pend_next = pn;
 
     TB_PHASE(3)
     // drop finished connections from the active lists; the next wake-up
     int64_t next = INT64_MAX;
-    if (!prune_later)
+    if (!KEEP)
     {
         int k = 0, n = hr.n_snd;
         for (int i = 0; i < n; i++)
@@ -277,7 +310,7 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
         }
         hr.n_snd = k;
     }
-    if (!prune_later)
+    if (!KEEP)
     {
         int k = 0, n = hr.n_rcv;
         for (int i = 0; i < n; i++)
@@ -296,24 +329,24 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
     }
     if (pst < next)
         next = pst;
-    hr.wake = nic.size > 0 ? t + 1 : (next == INT64_MAX ? INT64_MAX : next / SLOT_PS);
+    hr.wake = held > 0 ? t + 1 : (next == INT64_MAX ? INT64_MAX : next / SLOT_PS);
     *wake = hr.wake;
     TB_PHASE(4)
     // counters
-    ev_add(s, hr.world, EV_DROPS, nic.drops);
-    ev_add(s, hr.world, EV_MARKS, nic.marks);
+    ev_add(s, hr.world, EV_DROPS, drops);
+    ev_add(s, hr.world, EV_MARKS, marks);
     ev_add(s, hr.world, EV_RETX, c.retx);
     ev_add(s, hr.world, EV_RTO, c.rtos);
     ev_add(s, hr.world, EV_HOST_PKT, c.pkts);
     ev_add(s, hr.world, EV_HOST_SND, c.snd_pkts);
-    ev_add(s, hr.world, EV_HOST_FRAMES, nic.offered);
+    ev_add(s, hr.world, EV_HOST_FRAMES, offered);
     ev_add(s, hr.world, EV_OVF_RING, c.ovf);
-    ev_add(s, hr.world, EV_OVF_TX, nic.ovf);
+    ev_add(s, hr.world, EV_OVF_TX, ovf);
     ev_add(s, hr.world, EV_TIES, ties);
     *ties_out += ties;
     *done_out += c.done;
     TB_PHASE(5)
-    return nic.n_out > 0 || nic.size > 0;
+    return sent > 0 || held > 0;
 }
 
 // ------------------------------------------------------------------ switches

@@ -57,10 +57,13 @@ struct alignas(16) SndCore
     // read-only
     uint64_t it_off;
     int world, src_local, dst_local;
-    uint32_t hash_data, hash_ack;
     int m_first, m_cnt; // messages (global ids, consecutive)
     uint32_t it_cap;    // sent-list / RTT-history ring capacity
-    uint32_t pad0[2];
+    uint32_t up;        // its data's ECMP choice: hash_data modulo the world's equal-cost uplinks
+    // (while an event works on the core; 0 in memory) the flag word of the sent list stored last, its
+    // number + 1 and its value
+    uint32_t cw_at, cw;
+    uint32_t pad0;
     // application and socket
     int m_due, m_wr, m_dn;
     uint8_t st, cong, fin, fin_on;
@@ -80,6 +83,7 @@ struct alignas(16) SndCore
 };
 struct SndRec : SndCore
 {
+    uint32_t hash_data, hash_ack;
     // TcpCubic
     uint32_t cub_cnt, cub_lastmax, cub_origin, cub_endseq, cub_samples, cub_ackcnt, cub_tcpcwnd;
     uint8_t cub_found, pad1[3];
@@ -97,7 +101,8 @@ struct alignas(16) RcvCore
     uint32_t hash_ack;
     uint32_t oo_cap;
     uint32_t bytes;             // the connection's bytes (all its messages)
-    uint32_t pad0[4];
+    uint32_t up_ack;            // its ACKs' ECMP choice
+    uint32_t pad0[3];
     uint8_t fin_on, up, est, st;
     uint32_t rcv_nxt, ooo_n, ooo_h, prior_rcv_nxt;
     uint8_t last_n, syn_n, delack_count, ce_state, prior_flag, reserved, ecn_r, pad1;

@@ -28,13 +28,14 @@ struct SwShared
     unsigned tied;          // egress ports with arrivals at one instant
     int cap;
     // the arrays after this header, addressed from the scratch itself (so that the compiler keeps
-    // them in the shared address space): the staged frames [cap], two words and a half-word per
-    // frame (word arrays padded to four entries)
+    // them in the shared address space): a host's offered frames [OUT_FRAMES], the staged frames
+    // [cap], two words, a half-word and a byte per frame (padded to four entries)
     TB_D unsigned char *bytes() { return reinterpret_cast<unsigned char *>(this); }
     TB_D const unsigned char *bytes() const { return reinterpret_cast<const unsigned char *>(this); }
-    TB_D Frame *fr() { return reinterpret_cast<Frame *>(bytes() + header()); }
-    TB_D const Frame *fr() const { return reinterpret_cast<const Frame *>(bytes() + header()); }
-    TB_D uint32_t *key() { return reinterpret_cast<uint32_t *>(bytes() + header() + (size_t)cap * sizeof(Frame)); }
+    TB_D Frame *offered() { return reinterpret_cast<Frame *>(bytes() + header()); }
+    TB_D Frame *fr() { return offered() + OUT_FRAMES; }
+    TB_D const Frame *fr() const { return const_cast<SwShared *>(this)->fr(); }
+    TB_D uint32_t *key() { return reinterpret_cast<uint32_t *>(fr() + cap); }
     TB_D uint32_t *mem() { return key() + pad4(cap); }
     TB_D uint16_t *src() { return reinterpret_cast<uint16_t *>(mem() + pad4(cap)); }
     TB_D uint8_t *out() { return reinterpret_cast<uint8_t *>(src() + pad4(cap)); }
@@ -43,7 +44,7 @@ struct SwShared
     TB_D bool due_fit(size_t bytes) const { return (size_t)pad4(cap) * 8 >= bytes; }
     // (unstaged) [ingress][egress] counts, then offsets, in place of the staged frames
     typedef int Row[33];
-    TB_D Row *rows() { return reinterpret_cast<Row *>(bytes() + header()); }
+    TB_D Row *rows() { return reinterpret_cast<Row *>(fr()); }
     static TB_HDI size_t header();
     static TB_HDI int pad4(int n);
 };
@@ -54,7 +55,7 @@ TB_HDI int SwShared::pad4(int n) { return (n + 3) & ~3; }
 TB_HDI size_t sw_shared_bytes(int cap)
 {
     const size_t staged = (size_t)cap * sizeof(Frame) + (size_t)SwShared::pad4(cap) * 11, rows = 32 * sizeof(SwShared::Row);
-    return SwShared::header() + (((staged > rows ? staged : rows) + 15) & ~(size_t)15);
+    return SwShared::header() + OUT_FRAMES * sizeof(Frame) + (((staged > rows ? staged : rows) + 15) & ~(size_t)15);
 }
 // a warp's scratch at `p` (every lane may call it: the same value is written)
 TB_D SwShared *sw_shared_at(unsigned char *p, int cap)

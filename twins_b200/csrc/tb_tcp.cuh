@@ -21,14 +21,22 @@ struct Due
     int kind; // 0 retransmission, 1 delayed ACK, 2 SYN or deferred send, 3 SYN-ACK, 4 LAST_ACK, 5 FIN+ACK
 };
 
-// one host's slot: its egress, the running event's chain, the timers due, counters
+// one host's slot: the frames offered to its NIC so far, the running event's chain, the timers due,
+// counters
 struct HostCtx
 {
     const Sim *s;
     const WorldDesc *wd;
     int h;
     bool dctcp, cubic;
-    Egress nic;
+    // the host's sending end: with a warp of its own, the frames offered go to a list that is played
+    // through the NIC; hosts that share a warp enqueue each (the list cost them 5-10%)
+    bool list;
+    HostNic *nic;
+    Frame *out; // [OUT_FRAMES], out_n of them offered and not yet played
+    int out_n;
+    Egress eg;
+    int64_t kicked; // the instant of a ScheduleNow'd event being handled (-1: none)
     Chain ech;
     Due *due; // [DUE_CAP], beside the context: an array indexed at run time would keep all of it in memory
     int nd, di;
@@ -37,13 +45,23 @@ struct HostCtx
     unsigned long long pkts, snd_pkts;
 };
 
-// A connection's record while an event works on it: its core in registers (a record worked on in
+// A connection's record while events work on it: its core in registers (a record worked on in
 // place is read and written through memory field by field, since the compiler cannot tell it from
-// the rings and frames the event stores), the rest of it behind `rec`.
+// the rings and frames the event stores), the rest of it behind `rec`. With one host per warp the
+// sender's and the receiver's record last used stay in registers from event to event (Recs): most of
+// a busy host's events in a slot are one connection's, and loading a record that the event before
+// has just stored waits 600 cycles for the stores.
 struct Snd : SndCore
 {
     SndRec *rec;
-    TB_D explicit Snd(SndRec &r) : rec(&r) { load_core<SndCore>(this, &r); }
+    int f; // the connection (-1: none)
+    TB_D Snd() : f(-1) {}
+    TB_D void load(SndRec &r, int flow)
+    {
+        rec = &r;
+        f = flow;
+        load_core<SndCore>(this, &r);
+    }
     TB_D void store() const { store_core<SndCore>(rec, this); }
     // a core from its record
     template <class Core>
@@ -71,11 +89,64 @@ struct Snd : SndCore
 struct Rcv : RcvCore
 {
     RcvRec *rec;
-    TB_D explicit Rcv(RcvRec &r) : rec(&r) { Snd::load_core<RcvCore>(this, &r); }
+    int f;
+    TB_D Rcv() : f(-1) {}
+    TB_D void load(RcvRec &r, int flow)
+    {
+        rec = &r;
+        f = flow;
+        Snd::load_core<RcvCore>(this, &r);
+    }
     TB_D void store() const { Snd::store_core<RcvCore>(rec, this); }
 };
 static_assert(offsetof(SndCore, m_due) == REC_FIXED && offsetof(RcvCore, fin_on) == REC_FIXED && sizeof(SndCore) % 16 == 0 && sizeof(RcvCore) % 16 == 0,
               "cores move as 16-byte words");
+
+template <bool KEEP>
+struct Recs
+{
+    Snd S;
+    Rcv R;
+    TB_D Snd &snd(const Sim &s, int f)
+    {
+        if (!KEEP || S.f != f)
+        {
+            if (KEEP && S.f >= 0)
+                S.store();
+            S.load(s.snd[f], f);
+        }
+        return S;
+    }
+    TB_D Rcv &rcv(const Sim &s, int f)
+    {
+        if (!KEEP || R.f != f)
+        {
+            if (KEEP && R.f >= 0)
+                R.store();
+            R.load(s.rcv[f], f);
+        }
+        return R;
+    }
+    // after an event of the one or the other: the record stays, or goes back to memory
+    TB_D void snd_done() const
+    {
+        if (!KEEP)
+            S.store();
+    }
+    TB_D void rcv_done() const
+    {
+        if (!KEEP)
+            R.store();
+    }
+    TB_D void flush()
+    {
+        if (S.f >= 0)
+            S.store();
+        if (R.f >= 0)
+            R.store();
+        S.f = R.f = -1;
+    }
+};
 
 // a timer armed during the slot that falls due before its end joins the slot's timers, after the
 // ones of its time already there (reference: due_insert, src/step.cuh:342-360)
@@ -95,10 +166,18 @@ TB_D void timer_in_slot(HostCtx &c, int64_t at, int f, int kind)
 }
 
 // ------------------------------------------------------------------ frames out
+// the offered frames through the NIC, and its starts by `until` (an offset in the slot)
+TB_DN void nic_run(HostNic *nic, Frame *list, int n, int until)
+{
+    HostNic q = *nic; // (in registers)
+    q.run_list(list, n, until);
+    *nic = q;
+}
+
 // a segment leaves the socket for the host's device queue: data carry their sequence number, the
 // others their acknowledgement; the ECMP uplink is the direction's flow hash (reference: emit,
 // src/step.cuh:368-384)
-TB_D void to_device(HostCtx &c, int f, uint8_t flags, uint32_t num, uint16_t wire_len, bool toward_sender, uint32_t hash, int dst,
+TB_D void to_device(HostCtx &c, int f, uint8_t flags, uint32_t num, uint16_t wire_len, bool toward_sender, uint32_t up, int dst,
                     int64_t now)
 {
     Frame fr;
@@ -109,17 +188,30 @@ TB_D void to_device(HostCtx &c, int f, uint8_t flags, uint32_t num, uint16_t wir
     fr.dst = (uint16_t)dst;
     fr.flags = (uint8_t)(flags | (c.dctcp ? F_ECT : 0));
     fr.to_sender = toward_sender ? 1 : 0;
-    fr.up = (uint16_t)(hash % (uint32_t)c.wd->ecmp_n);
+    fr.up = (uint16_t)up;
     fr.ch = c.ech;
-    c.nic.enqueue(fr, now);
+    if (!c.list)
+    {
+        c.eg.kicked = c.kicked;
+        c.eg.enqueue(fr, now);
+        return;
+    }
+    if (c.out_n == OUT_FRAMES)
+    {
+        // (a full list: the NIC takes it now; what it starts later in the slot it starts the same)
+        nic_run(c.nic, c.out, c.out_n, (int)(now - c.nic->S0));
+        c.out_n = 0;
+    }
+    fr.to_sender |= c.kicked == now ? OFFER_KICK : 0;
+    frame_copy(&c.out[c.out_n++], &fr);
 }
 TB_D void emit_snd(HostCtx &c, int f, const SndCore &S, uint8_t flags, uint32_t num, uint16_t wire_len, int64_t now)
 {
-    to_device(c, f, flags, num, wire_len, false, S.hash_data, S.dst_local, now);
+    to_device(c, f, flags, num, wire_len, false, S.up, S.dst_local, now);
 }
 TB_D void emit_rcv(HostCtx &c, int f, const RcvCore &R, uint8_t flags, uint32_t ack, uint16_t len, int64_t now)
 {
-    to_device(c, f, flags, ack, len, true, R.hash_ack, R.src_local, now);
+    to_device(c, f, flags, ack, len, true, R.up_ack, R.src_local, now);
 }
 
 // the receiver's pure ACK (SendEmptyPacket): ECE while it owes the sender an echo of CE, unless this
@@ -172,6 +264,16 @@ struct SentList
     uint32_t *fw; // flag words
     uint32_t cap;
 
+    // A flag word, and its store. The word stored last is kept with the record's core: an append reads
+    // the word that the append before it stored, and a load of a line just stored waits for the store.
+    TB_D uint32_t word(uint32_t w) const { return w + 1 == S.cw_at ? S.cw : fw[w]; }
+    TB_D void set_word(uint32_t w, uint32_t v)
+    {
+        fw[w] = v;
+        S.cw_at = w + 1;
+        S.cw = v;
+    }
+
     TB_D SentList(const Sim &s, SndCore &S_) : S(S_)
     {
         start = s.it_start + S.it_off;
@@ -189,13 +291,13 @@ struct SentList
     TB_D static uint32_t spread(uint8_t f) { return (f & 1u) | (f & 2u) << 7 | (f & 4u) << 14; } // (flag bits -> plane bits)
     TB_D uint8_t flags_at(uint32_t p) const
     {
-        const uint32_t w = fw[p >> 3] >> (p & 7);
+        const uint32_t w = word(p >> 3) >> (p & 7);
         return (uint8_t)((w & 1u) | (w >> 7 & 2u) | (w >> 14 & 4u));
     }
     TB_D void write_at(uint32_t p, uint8_t f)
     {
         const uint32_t b = p & 7;
-        fw[p >> 3] = (fw[p >> 3] & ~(0x010101u << b)) | spread(f) << b;
+        set_word(p >> 3, (word(p >> 3) & ~(0x010101u << b)) | spread(f) << b);
     }
     TB_D uint8_t flags(uint32_t i) const { return flags_at(pos(i)); }
     TB_D static bool candidate(uint8_t f) { return (f & (FL_LOST | FL_RETX | FL_SACK)) == FL_LOST; }
@@ -243,7 +345,7 @@ struct SentList
         uint32_t w = p0 >> 3, carry = 0;
         for (bool first = true;; first = false)
         {
-            const uint32_t x = fw[w];
+            const uint32_t x = word(w);
             uint32_t y = ((x << 1) & 0xFEFEFEu) | carry;
             carry = (x >> 7) & 0x010101u;
             if (first)
@@ -254,10 +356,10 @@ struct SentList
             if (--words == 0)
             {
                 const uint32_t mine = ((2u << (pe & 7)) - 1) * 0x010101u;
-                fw[w] = (y & mine) | (x & ~mine);
+                set_word(w, (y & mine) | (x & ~mine));
                 return;
             }
-            fw[w] = y;
+            set_word(w, y);
             w = next_word(w);
         }
     }
@@ -270,8 +372,8 @@ struct SentList
         uint32_t w = p0 >> 3;
         for (bool first = true;; first = false)
         {
-            const uint32_t x = fw[w];
-            const uint32_t nx = words == 1 ? 0u : fw[next_word(w)];
+            const uint32_t x = word(w);
+            const uint32_t nx = words == 1 ? 0u : word(next_word(w));
             uint32_t y = ((x >> 1) & 0x7F7F7Fu) | ((nx & 0x010101u) << 7);
             if (first)
             {
@@ -281,10 +383,10 @@ struct SentList
             if (--words == 0)
             {
                 const uint32_t mine = ((2u << (pe & 7)) - 1) * 0x010101u;
-                fw[w] = (y & mine) | (x & ~mine);
+                set_word(w, (y & mine) | (x & ~mine));
                 return;
             }
-            fw[w] = y;
+            set_word(w, y);
             w = next_word(w);
         }
     }
@@ -307,7 +409,7 @@ struct SentList
         const uint32_t p = pos(i);
         start[p] = seq;
         if (i == S.it_n && !(p & 7) && S.it_n + 8 <= cap)
-            fw[p >> 3] = spread(f); // (an append opening a word whose other positions are all free: no read)
+            set_word(p >> 3, spread(f)); // (an append opening a word whose other positions are all free: no read)
         else
             write_at(p, f);
         S.sack_n += (f & FL_SACK) ? 1u : 0u;
@@ -347,7 +449,7 @@ struct SentList
                 run = cap - p;
             if (run > S.it_n - i)
                 run = S.it_n - i;
-            const uint32_t w = fw[p >> 3];
+            const uint32_t w = word(p >> 3);
             const uint32_t m = (want(w & 0xFFu, w >> 8 & 0xFFu, w >> 16 & 0xFFu) >> b) & ((1u << run) - 1);
             if (m)
                 return i + lowest(m);
@@ -408,7 +510,7 @@ TB_D void everything_lost(SentList &L)
     for (uint32_t i = 0; i < S.it_n;)
     {
         const uint32_t p = L.pos(i);
-        L.fw[p >> 3] = 0xFFu;
+        L.set_word(p >> 3, 0xFFu);
         i += 8 - (p & 7);
     }
     S.lost_b = S.cand_b = sent_bytes(S);
@@ -1520,18 +1622,19 @@ TB_D bool add_active(const Sim &s, int *list, int &n, int f, unsigned &ovf)
 }
 // a message's start time: the connection's first message opens it (SYN, the connection timeout
 // armed), a later one is written to the stream if the connection is up
-TB_D void app_event(HostCtx &c, HostRec &hr, int *act_snd, int m, int64_t now)
+template <bool KEEP>
+TB_D void app_event(HostCtx &c, Recs<KEEP> &q, HostRec &hr, int *act_snd, int m, int64_t now)
 {
     const WorldDesc &wd = *c.wd;
     const int f = c.s->msgs[m].conn;
-    Snd S(c.s->snd[f]);
+    Snd &S = q.snd(*c.s, f);
     if (S.m_first != m)
     {
         chain_msg_root(c.ech, m - wd.msg0);
         S.m_due++;
         if (S.st == S_EST)
             app_write(c, f, S, now);
-        S.store();
+        q.snd_done();
         return;
     }
     chain_app_root(c.ech, hr.local, f - wd.conn0);
@@ -1545,7 +1648,7 @@ TB_D void app_event(HostCtx &c, HostRec &hr, int *act_snd, int m, int64_t now)
     chain_child(S.rec->rchain, c.ech, code_lead(CONN_TO_PS));
     S.timing_time = now;
     emit_snd(c, f, S, F_SYN, 0, SYN_LEN, now);
-    S.store();
+    q.snd_done();
 }
 
 // ------------------------------------------------------------------ timers and frames
@@ -1610,18 +1713,17 @@ TB_D void rcv_timer(HostCtx &c, int f, Rcv &R, const Due &d, int64_t now)
         send_fin_ack(c, f, R, now);
     }
 }
-TB_D void timer_event(HostCtx &c, const Due &d, int64_t now)
+template <bool KEEP>
+TB_D void timer_event(HostCtx &c, Recs<KEEP> &q, const Due &d, int64_t now)
 {
     if (d.kind == 0 || d.kind == 2)
     {
-        Snd S(c.s->snd[d.flow]);
-        snd_timer(c, d.flow, S, d, now);
-        S.store();
+        snd_timer(c, d.flow, q.snd(*c.s, d.flow), d, now);
+        q.snd_done();
         return;
     }
-    Rcv R(c.s->rcv[d.flow]);
-    rcv_timer(c, d.flow, R, d, now);
-    R.store();
+    rcv_timer(c, d.flow, q.rcv(*c.s, d.flow), d, now);
+    q.rcv_done();
 }
 
 // a frame at its destination host: at the sender a SYN-ACK (connected: ACK, then the application's
@@ -1664,7 +1766,7 @@ TB_D void rcv_frame(HostCtx &c, HostRec &hr, int f, Rcv &R, const Frame &p, int6
         }
         if (R.est)
             return;
-        c.nic.kicked = now; // (the SYN's arrival ScheduleNow's CompleteFork)
+        c.kicked = now; // (the SYN's arrival ScheduleNow's CompleteFork)
         chain_child(c.ech, c.ech, CODE_NOW);
         send_synack(c, f, R, now);
         return;
@@ -1685,19 +1787,18 @@ TB_D void rcv_frame(HostCtx &c, HostRec &hr, int f, Rcv &R, const Frame &p, int6
             rcv_closed(R);
     }
 }
-TB_D void on_frame(HostCtx &c, HostRec &hr, const Frame &p, int64_t now)
+template <bool KEEP>
+TB_D void on_frame(HostCtx &c, Recs<KEEP> &q, HostRec &hr, const Frame &p, int64_t now)
 {
     const int f = (int)p.flow;
     if (p.to_sender)
     {
-        Snd S(c.s->snd[f]);
-        snd_frame(c, f, S, p, now);
-        S.store();
+        snd_frame(c, f, q.snd(*c.s, f), p, now);
+        q.snd_done();
         return;
     }
-    Rcv R(c.s->rcv[f]);
-    rcv_frame(c, hr, f, R, p, now);
-    R.store();
+    rcv_frame(c, hr, f, q.rcv(*c.s, f), p, now);
+    q.rcv_done();
 }
 
 } // namespace tb
