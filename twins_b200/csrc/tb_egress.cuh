@@ -85,10 +85,25 @@ TB_D void ev_add(const Sim &s, int world, int i, unsigned long long n)
 
 // link messages: slot `slot` of link `link`
 TB_D size_t msg_index(const Sim &s, int64_t slot, int link) { return (size_t)(slot & (NB - 1)) * s.L + link; }
-TB_D int msg_count(const Sim &s, int64_t slot, int link)
+// Its frames and how many of them arrive in the slot after it, the first ones; the others arrive in the
+// next. The sender, which knows the arrival times, says so in the tag, so that a reader takes the
+// frames of its slot and no others: the late ones of the message before last, the early ones of the last.
+struct MsgTag
 {
-    int64_t v = tag_load(&s.msg_tag[msg_index(s, slot, link)]);
-    return (v >> 16) == slot ? (int)(v & 0xFFFF) : 0;
+    int n, early;
+};
+TB_D MsgTag msg_tag(const Sim &s, int64_t slot, int link)
+{
+    const int64_t v = slot >= 0 ? tag_load(&s.msg_tag[msg_index(s, slot, link)]) : -1;
+    MsgTag m = {0, 0};
+    if (slot >= 0 && (v >> 20) == slot)
+        m = {(int)(v & 1023), (int)(v >> 10 & 1023)};
+    return m;
+}
+static_assert(MAX_TX < 1024, "a tag's counts");
+TB_D void msg_seal(const Sim &s, int64_t slot, int link, int n, int early)
+{
+    tag_store(&s.msg_tag[msg_index(s, slot, link)], slot << 20 | (int64_t)early << 10 | n);
 }
 TB_D const Frame *msg_frames(const Sim &s, int64_t slot, int link) { return s.msg + msg_index(s, slot, link) * MAX_TX; }
 
@@ -138,7 +153,7 @@ struct Egress
     int64_t kicked;     // the instant of a ScheduleNow'd event being handled (-1: none)
     int64_t idle_began; // the last start this slot on an idle wire (-1: none)
     Frame *msg;
-    int n_out;
+    int n_out, early; // frames started, of which the first `early` arrive in the next slot
     unsigned drops, marks, ovf, offered;
 #ifdef TB_QTRACE
     const Sim *qs; // the trace's sink; the queue's ns-3 node and device
@@ -160,7 +175,7 @@ struct Egress
         horizon = horizon_;
         kicked = idle_began = -1;
         msg = msg_;
-        n_out = 0;
+        n_out = early = 0;
         drops = marks = ovf = offered = 0;
     }
 
@@ -193,6 +208,7 @@ struct Egress
             busy_until = t1;
             o.ts = t1 + PROP_PS;
             frame_store_link(&msg[n_out++], o);
+            early += t1 < horizon; // (PROP_PS is a slot)
             head = head + 1 == cap ? 0 : head + 1;
         }
     }
@@ -269,7 +285,7 @@ struct HostNic
     int64_t S0;
     Frame *msg;
     Chain *wire;         // the chain of the frame on the wire
-    int n_out;
+    int n_out, early;
     unsigned drops, marks, ovf, offered;
     int node;
 
@@ -295,7 +311,7 @@ struct HostNic
         qcap = wd.qcap;
         msg = msg_;
         wire = &hr.last;
-        n_out = 0;
+        n_out = early = 0;
         drops = marks = ovf = offered = 0;
         node = hr.local;
     }
@@ -351,6 +367,7 @@ struct HostNic
                 f.ts = S0 + busy + PROP_PS;
                 f.to_sender &= 1;
                 frame_store_link(&msg[n_out++], f);
+                early += busy < SLOT;
                 if (!start)
                 {
                     i++;

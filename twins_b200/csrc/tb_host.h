@@ -22,7 +22,12 @@ namespace tb
 constexpr int SW_STAGE = 192;
 constexpr int SW_STAGE_MAX = TB_CHAIN_RUNS > 9 ? 256 : 384; // (what four warps' scratch fits in 227 KB)
 constexpr int SW_STAGE_SMALL = 96;
-constexpr int SW_STAGE_TWO = 288; // the most with which two blocks of four warps fit on an SM
+constexpr int SW_STAGE_TWO = 288; // two blocks of four warps fit on an SM with it
+
+// The staging area of a launch shape's `stage` frames. A shape counts the frames of two slots' link
+// messages, of which a reader takes about half (the late frames of the one, the early ones of the
+// other); the area holds three quarters of them.
+inline int stage_area(int stage) { return stage * 3 / 4 > 1 ? stage * 3 / 4 : 1; }
 
 // the grid of a launch: a block per `warps` units, at most what is co-resident (per_sm blocks on
 // each of sms SMs; 0: the shape does not fit), or the caller's grid when it asked for one

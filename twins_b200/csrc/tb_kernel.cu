@@ -255,7 +255,7 @@ template <bool MANY>
 __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t t, int lane, SwShared &sh, unsigned &ties,
                                           unsigned *done_sink)
 {
-    int h, w = 0, n2 = -1, n1 = -1, due_n = 0, due_ovf = 0;
+    int h, w = 0, first2 = 0, n2 = 0, n1 = 0, due_n = 0, due_ovf = 0;
     int64_t t0 = 0;
     bool run = false;
     const Frame *stage = nullptr;
@@ -266,8 +266,10 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
         const HostRec &hr = s.hosts[h];
         w = hr.world;
         const int link = hr.in_link;
-        n2 = t >= 2 ? msg_count(s, t - 2, link) : 0;
-        n1 = t >= 1 ? msg_count(s, t - 1, link) : 0;
+        const MsgTag a2 = msg_tag(s, t - 2, link), a1 = msg_tag(s, t - 1, link);
+        first2 = a2.early;
+        n2 = a2.n - a2.early;
+        n1 = a1.early;
         const int n = n2 + n1;
         const int64_t next = world_next(s, w);
         t0 = world_t0(s, w);
@@ -282,7 +284,7 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
         const bool staged = n <= sh.cap;
         if (staged)
             for (int i = lane; i < n; i += 32)
-                frame_load_link(sh.fr()[i], i < n2 ? msg_frames(s, t - 2, link) + i : msg_frames(s, t - 1, link) + (i - n2));
+                frame_load_link(sh.fr()[i], i < n2 ? msg_frames(s, t - 2, link) + first2 + i : msg_frames(s, t - 1, link) + (i - n2));
         __syncwarp();
         const bool cubic = s.worlds[w].cc == CC_CUBIC;
         if (staged)
@@ -352,9 +354,11 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
                 // the connections of its first arrivals into L1 (the lanes' event loops diverge
                 // next, and would each wait for these one after the other)
                 const int link = hr.in_link;
-                n2 = t >= 2 ? msg_count(s, t - 2, link) : 0;
-                n1 = t >= 1 ? msg_count(s, t - 1, link) : 0;
-                const Frame *m2 = msg_frames(s, t - 2, link), *m1 = msg_frames(s, t - 1, link);
+                const MsgTag a2 = msg_tag(s, t - 2, link), a1 = msg_tag(s, t - 1, link);
+                first2 = a2.early;
+                n2 = a2.n - a2.early;
+                n1 = a1.early;
+                const Frame *m2 = msg_frames(s, t - 2, link) + first2, *m1 = msg_frames(s, t - 1, link);
                 for (int j = 0; j < 4 && j < n2 + n1; j++)
                 {
                     const Frame *f = j < n2 ? &m2[j] : &m1[j - n2];
@@ -372,7 +376,7 @@ __device__ __forceinline__ void host_unit(const Sim &s, int h0, int nh, int64_t 
     bool act = false;
     if (run)
     {
-        act = host_step<!MANY>(s, h, t - t0, t, &wake, &ties, &done, sh.offered(), stage, n2, n1, due, due_n, due_ovf);
+        act = host_step<!MANY>(s, h, t - t0, t, &wake, &ties, &done, sh.offered(), stage, first2, n2, n1, due, due_n, due_ovf);
         if constexpr (MANY)
             host_report(s, w, t0, act, wake, done);
     }
@@ -399,7 +403,10 @@ __device__ __noinline__ bool switch_unstaged(const SwCtx &x, SwShared &sh, int l
 {
     const bool on = lane < x.sr->k;
     if (on)
-        c.pk = sw_phase_window(x, sh, lane);
+    {
+        sw_phase_clear(x, sh, lane);
+        c.pk = (unsigned)input_of(x, sh, lane).count();
+    }
     __syncwarp();
     if (x.spray)
     {
@@ -430,7 +437,7 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
     const int64_t next = world_next(s, sr.world), t0 = world_t0(s, sr.world);
     const int k = sr.k;
     const bool on = lane < k;
-    int link = -1, n2 = 0, n1 = 0, qn = 0, qh = 0;
+    int link = -1, first2 = 0, n2 = 0, n1 = 0, qn = 0, qh = 0;
     if (on)
     {
         const PortRec &pr = s.ports[sr.port0 + lane];
@@ -439,8 +446,10 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
         qh = pr.q_head;
         if (link >= 0)
         {
-            n2 = gt >= 2 ? msg_count(s, gt - 2, link) : 0;
-            n1 = gt >= 1 ? msg_count(s, gt - 1, link) : 0;
+            const MsgTag a2 = msg_tag(s, gt - 2, link), a1 = msg_tag(s, gt - 1, link);
+            first2 = a2.early;
+            n2 = a2.n - a2.early;
+            n1 = a1.early;
         }
     }
     // its world does not run this slot; or no frame arriving and every queue empty: nothing to do
@@ -469,8 +478,9 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
             incl += v;
     }
     const int total = __shfl_sync(FULL, incl, 31), first = incl - n2 - n1;
-    sh.raw2[lane] = n2;
-    sh.raw1[lane] = n1;
+    sh.win[lane][0] = first2;
+    sh.win[lane][1] = first2 + n2;
+    sh.win[lane][2] = n1;
     sh.link[lane] = link;
     sh.cnt[lane] = 0;
     bool act;
@@ -479,10 +489,10 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
         uint32_t *key = sh.key(), *mem = sh.mem();
         uint16_t *src = sh.src();
         uint8_t *out = sh.out();
-        const int64_t S0 = x.t * SLOT_PS, E0 = S0 + SLOT_PS;
+        const int64_t S0 = x.t * SLOT_PS;
         // each staged frame's port (5 bits) and place in its message (9 bits, 1: of msg[t-1])
         for (int j = 0; j < n2 + n1; j++)
-            src[first + j] = (uint16_t)(j < n2 ? lane << 10 | j : lane << 10 | 0x200 | (j - n2));
+            src[first + j] = (uint16_t)(j < n2 ? lane << 10 | (first2 + j) : lane << 10 | 0x200 | (j - n2));
         if (lane == 0)
             sh.tied = 0;
         // the queue's next frames, which the slot starts (a slot sends 8 full frames), into L1
@@ -493,7 +503,8 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
                 prefetch_l1(&ring[qh + j < s.ring ? qh + j : qh + j - s.ring], sizeof(Frame));
         }
         __syncwarp();
-        // the frames: copied, their place in the window
+        c.pk = n2 + n1;
+        // the frames: copied, their keys
         for (int i = lane; i < total; i += 32)
         {
             const int v = src[i], q = v >> 10, l = sh.link[q];
@@ -501,18 +512,12 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
             Frame f;
             frame_load_link(f, msg_frames(s, m1 ? gt - 1 : gt - 2, l) + (v & 0x1FF));
             frame_copy(&sh.fr()[i], &f);
-            const bool in = m1 ? f.ts < E0 : f.ts >= S0;
-            c.pk += in;
-            uint32_t ky = ~0u;
-            if (in)
+            uint32_t ky = (uint32_t)(f.ts - S0);
+            if (x.spray)
             {
-                ky = (uint32_t)(f.ts - S0);
-                if (x.spray)
-                {
-                    const int ep = x.wd->n_fail ? epoch_of(*x.wd, f.ts) : 0;
-                    const bool draws = !port_down(*x.wd, sr.local, q, ep) && routes_to(*x.wd, sr.local, f.dst, ep) > 0;
-                    ky = ky << 12 | (uint32_t)(2047 - f.len) << 1 | (draws ? 0u : 1u);
-                }
+                const int ep = x.wd->n_fail ? epoch_of(*x.wd, f.ts) : 0;
+                const bool draws = !port_down(*x.wd, sr.local, q, ep) && routes_to(*x.wd, sr.local, f.dst, ep) > 0;
+                ky = ky << 12 | (uint32_t)(2047 - f.len) << 1 | (draws ? 0u : 1u);
             }
             key[i] = ky;
         }
@@ -526,7 +531,7 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
 #endif
         if (x.spray)
         {
-            sw_spray_staged(x, sh, lane, total, first, first + n2, g_rng_ahead, c.ties);
+            sw_spray_staged(x, sh, lane, total, first, first + n2 + n1, g_rng_ahead, c.ties);
             __syncwarp();
         }
 #ifdef TB_PROFILE
@@ -537,15 +542,11 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
         // each frame's egress port
         for (int i = lane; i < total; i += 32)
         {
-            int e = -1;
-            if (key[i] != ~0u)
-            {
-                e = sw_egress_for(x, sh.fr()[i], src[i] >> 10, x.spray ? out[i] : 0);
-                if (e < 0)
-                    c.drops++;
-                else
-                    atomicAdd(&sh.cnt[e], 1);
-            }
+            const int e = sw_egress_for(x, sh.fr()[i], src[i] >> 10, x.spray ? out[i] : 0);
+            if (e < 0)
+                c.drops++;
+            else
+                atomicAdd(&sh.cnt[e], 1);
             out[i] = (uint8_t)e;
         }
         __syncwarp();
@@ -567,12 +568,12 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
             if (e >= 0)
                 mem[sh.base[e] + atomicSub(&sh.cnt[e], 1) - 1] = (x.spray ? key[i] >> 12 : key[i]) << 9 | (uint32_t)i;
         }
-        sh.raw2[lane] = n;
+        sh.num[lane] = n;
         __syncwarp();
         for (int j = lane; j < kept; j += 32)
         {
             const uint32_t v = mem[j];
-            const int e = out[v & 511], b = sh.base[e], m = sh.raw2[e];
+            const int e = out[v & 511], b = sh.base[e], m = sh.num[e];
             int rank = 0, same = 0;
             for (int i = b; i < b + m; i++)
             {
@@ -894,7 +895,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
 }
 
 // dynamic shared memory of a block: one switch scratch (with its staging area) per warp
-static size_t smem_bytes(int stage_cap) { return sw_shared_bytes(stage_cap) * WARPS_PER_BLOCK; }
+static size_t smem_bytes(int stage_cap) { return sw_shared_bytes(stage_area(stage_cap)) * WARPS_PER_BLOCK; }
 
 // the instantiation of a launch shape: several hosts per warp or one host per warp; each with the
 // grid barrier or without (F_*: batches)
@@ -982,7 +983,8 @@ int launch_slots(const Sim &s, int grid, int max_slots_per_launch, int host_lane
     const int k = kind_of(host_lanes);
     if (!smem_attr(k) || stage_cap < 1 || stage_cap > SW_STAGE_MAX)
         return (int)cudaErrorInvalidValue;
-    void *args[] = {(void *)&s, (void *)&max_slots_per_launch, (void *)&host_lanes, (void *)&stage_cap};
+    int area = stage_area(stage_cap);
+    void *args[] = {(void *)&s, (void *)&max_slots_per_launch, (void *)&host_lanes, (void *)&area};
     return launch_kind(k, args, grid, stage_cap, stream);
 }
 
@@ -996,7 +998,8 @@ int launch_free(const Sim &s, int grid, int slots_per_world, int host_lanes, int
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return (int)e;
-    void *args[] = {(void *)&s, (void *)&host_lanes, (void *)&stage_cap};
+    int area = stage_area(stage_cap);
+    void *args[] = {(void *)&s, (void *)&host_lanes, (void *)&area};
     return launch_kind(k, args, grid, stage_cap, stream);
 }
 

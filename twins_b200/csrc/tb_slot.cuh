@@ -42,9 +42,8 @@ TB_D bool rcv_idle_for_good(const RcvRec &R)
 // One slot of host h. Returns true if it sent or holds frames; *wake: the next slot it must run.
 // t: the world's own slot (time); gt: the launch's slot, which indexes the link messages (equal
 // in a batch; a world that joins a running launch starts its own time at a later launch slot).
-// `stage`: the host's link messages of slots gt-2 and gt-1 copied to shared memory by its warp
-// (msg[gt-2] then msg[gt-1], n2 and n1 frames as their tags count), or null to read them in place
-// (n2, n1 < 0: read the tags).
+// Its arrivals: n2 frames of msg[gt-2] from frame first2 on, then the first n1 of msg[gt-1]; `stage`: copied
+// to shared memory by its warp, or null to read them in place.
 // KEEP (one host per warp): the records last used stay in registers between events (Recs); the active
 // lists are left unpruned and *wake counts only the host's queue and its next application start; the
 // caller prunes them (prune_lists_warp) and lowers the wake-up to the earliest timer of the
@@ -54,36 +53,21 @@ TB_D bool rcv_idle_for_good(const RcvRec &R)
 // `out` (KEEP): the list of the frames its events offer, room for OUT_FRAMES.
 template <bool KEEP>
 TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, unsigned *ties_out, unsigned *done_out, Frame *out,
-                    const Frame *stage = nullptr, int n2 = -1, int n1 = -1, Due *due = nullptr,
+                    const Frame *stage, int first2, int n2, int n1, Due *due = nullptr,
                     int due_n = 0, int due_ovf = 0)
 {
     const int64_t S0 = t * SLOT_PS, E0 = S0 + SLOT_PS;
     TB_PHASE_START
     HostRec &hr = s.hosts[h];
-    const int link = hr.in_link;
-    const Frame *m2 = nullptr, *m1 = nullptr;
+    const Frame *m2 = stage ? stage : msg_frames(s, gt - 2, hr.in_link) + first2, *m1 = stage ? stage + n2 : msg_frames(s, gt - 1, hr.in_link);
     int i2 = 0, i1 = 0;
-    auto ts_at = [&](const Frame *m, int j) { return stage ? m[j].ts : ts_load_link(&m[j]); };
     auto frame_at = [&](Frame &d, const Frame *m, int j) {
         if (stage)
             d = m[j];
         else
             frame_load_link(d, &m[j]);
     };
-    if (n2 < 0)
-        n2 = gt >= 2 ? msg_count(s, gt - 2, link) : 0;
-    if (n1 < 0)
-        n1 = gt >= 1 ? msg_count(s, gt - 1, link) : 0;
-    if (n2 > 0)
-    {
-        m2 = stage ? stage : msg_frames(s, gt - 2, link);
-        while (i2 < n2 && ts_at(m2, i2) < S0)
-            i2++;
-    }
-    if (n1 > 0)
-        m1 = stage ? stage + n2 : msg_frames(s, gt - 1, link);
-    bool input = i2 < n2 || (n1 > 0 && ts_at(m1, 0) < E0);
-    if (!input && t < hr.wake && hr.q_size == 0)
+    if (n2 == 0 && n1 == 0 && t < hr.wake && hr.q_size == 0)
     {
         *wake = hr.wake;
         return false;
@@ -202,7 +186,7 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
                 frame_at(p, m2, i2);
                 have_p = true;
             }
-            else if (i1 < n1 && ts_at(m1, i1) < E0)
+            else if (i1 < n1)
             {
                 frame_at(p, m1, i1);
                 have_p = true;
@@ -267,13 +251,13 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
     if (KEEP)
         recs.flush();
     TB_PHASE(2)
-    int sent, held;
+    int sent, early, held;
     unsigned drops, marks, ovf, offered;
     if (KEEP)
     {
         nic_run(&nic, c.out, c.out_n, (int)SLOT_PS - 1);
         nic.close(hr);
-        sent = nic.n_out, held = nic.size;
+        sent = nic.n_out, early = nic.early, held = nic.size;
         drops = nic.drops, marks = nic.marks, ovf = nic.ovf, offered = nic.offered;
     }
     else
@@ -283,11 +267,11 @@ TB_D bool host_step(const Sim &s, int h, int64_t t, int64_t gt, int64_t *wake, u
         hr.q_size = c.eg.size;
         hr.link_free = c.eg.busy_until;
         hr.last_start = c.eg.began;
-        sent = c.eg.n_out, held = c.eg.size;
+        sent = c.eg.n_out, early = c.eg.early, held = c.eg.size;
         drops = c.eg.drops, marks = c.eg.marks, ovf = c.eg.ovf, offered = c.eg.offered;
     }
     TB_PHASE(8)
-    tag_store(&s.msg_tag[msg_index(s, gt, h)], (int64_t)gt << 16 | sent);
+    msg_seal(s, gt, h, sent, early);
     hr.pend_next = pn;
 
     TB_PHASE(3)

@@ -274,7 +274,7 @@ struct Sim
     int64_t *h_t;
     uint32_t *oo_s, *oo_e;
     Frame *msg;          // [NB][L][MAX_TX]
-    int64_t *msg_tag;    // [NB][L] slot << 16 | count (an old slot reads as empty)
+    int64_t *msg_tag;    // [NB][L] slot << 20 | frames of the next slot << 10 | frames (an old slot reads as empty)
     Rng *sw_rng;         // [S] (spraying worlds)
     uint8_t *sw_up;      // [S][kmax * 2 * MAX_TX] per-packet route choices (spraying)
     int64_t *sw_ts;      // [S][kmax * 2 * MAX_TX] egress sorting scratch

@@ -22,8 +22,8 @@ namespace tb
 struct SwShared
 {
     int base[32], cnt[32];
-    int win[32][3];         // (unstaged) each ingress port's window in its messages: (i2, n2, n1)
-    int raw2[32], raw1[32]; // frames in the port's msg[t-2] / msg[t-1]
+    int num[32];            // arrivals per egress port
+    int win[32][3];         // each ingress port's frames of the slot: msg[t-2] from the first to the second, msg[t-1] to the third
     int link[32];           // the port's ingress link
     unsigned tied;          // egress ports with arrivals at one instant
     int cap;
@@ -65,7 +65,7 @@ TB_D SwShared *sw_shared_at(unsigned char *p, int cap)
     return sh;
 }
 
-// (unstaged) ingress window of a port: the tail of msg[t-2] from S0 on, the head of msg[t-1] before E0
+// (unstaged) a port's frames of the slot: the late ones of msg[t-2], the early ones of msg[t-1]
 struct Input
 {
     const Frame *m2, *m1;
@@ -104,15 +104,15 @@ TB_D int sw_egress_for(const SwCtx &x, const Frame &f, int q, int up)
 
 // ------------------------------------------------------------------ staged slots
 // The spraying draws of a staged slot: one per forwarded packet, in the order the packets arrive at
-// the node (all ports merged). key[i] of a frame in the slot's window is its offset in the slot
-// (20 bits), 2047 - its length (11 bits; the longer of two simultaneous frames first) and whether it
-// draws nothing (1 bit), ~0 outside the window. A frame's place among the draws is the number of
+// the node (all ports merged). key[i] of a frame is its offset in the slot (20 bits), 2047 - its length
+// (11 bits; the longer of two simultaneous frames first) and whether it draws nothing (1 bit); ~0
+// fills the last four. pos .. end - 1: the frames of the lane's port. A frame's place among the draws is the number of
 // drawing frames with smaller keys: a frame per lane counts them, and every draw is computed at
 // once from the stream's state and its look-ahead rows. Where two frames' keys tie, the places come
 // from a merge of the ports' frames instead, a port per lane, in which the ties are decided by the
 // chains in port order. A merge of every slot took one warp-wide step per frame. Each frame's
 // choice goes to out[i]; the stream's state moves on by the slot's draws.
-__device__ void sw_spray_staged(const SwCtx &x, SwShared &sh, int lane, int total, int first, int first1, const RngAhead &ahead, unsigned &ties)
+__device__ void sw_spray_staged(const SwCtx &x, SwShared &sh, int lane, int total, int pos, int end, const RngAhead &ahead, unsigned &ties)
 {
     const unsigned FULL = 0xffffffffu;
     uint32_t *key = sh.key(), *place = sh.mem();
@@ -139,16 +139,6 @@ __device__ void sw_spray_staged(const SwCtx &x, SwShared &sh, int lane, int tota
     }
     if (__any_sync(FULL, tie))
     {
-        // a port per lane: its frames in the window lie together
-        int pos = 0, end = 0;
-        if (lane < x.sr->k)
-        {
-            const int n2 = sh.raw2[lane], n1 = sh.raw1[lane];
-            for (pos = first; pos < first + n2 && key[pos] == ~0u; pos++)
-                ;
-            for (end = first1; end < first1 + n1 && key[end] != ~0u; end++)
-                ;
-        }
         __syncwarp();
         uint32_t head = pos < end ? key[pos] >> 1 : ~0u;
         int run = 0;
@@ -195,7 +185,7 @@ __device__ void sw_spray_staged(const SwCtx &x, SwShared &sh, int lane, int tota
     for (int i = lane; i < total; i += 32)
     {
         uint32_t u = 0;
-        if (key[i] != ~0u && !(key[i] & 1))
+        if (!(key[i] & 1))
         {
             const Frame &f = sh.fr()[i];
             const uint32_t nr = (uint32_t)routes_to(wd, x.sr->local, f.dst, wd.n_fail ? epoch_of(wd, f.ts) : 0);
@@ -253,14 +243,14 @@ TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *
     const int port = x.sr->port0 + e, cap = s.ring, out_link = s.H + port;
     if (n == 0 && pr.q_size == 0)
     {
-        tag_store(&s.msg_tag[msg_index(s, x.gt, out_link)], x.gt << 16);
+        msg_seal(s, x.gt, out_link, 0, 0);
         return false;
     }
     const int red_k = pr.red_k, qcap = pr.qcap;
     const int64_t S0 = x.t * SLOT_PS;
     Frame *ring = s.port_ring + (size_t)port * cap;
     Frame *msg = s.msg + msg_index(s, x.gt, out_link) * MAX_TX;
-    int head = pr.q_head, size = pr.q_size, n_out = 0;
+    int head = pr.q_head, size = pr.q_size, n_out = 0, early = 0;
     // the wire: busy until `busy` with a frame of tx_len bytes that began at `began` (a wire free
     // since before the slot: only that it is matters)
     int busy = -1, began = -SLOT, tx_len = 0;
@@ -334,6 +324,7 @@ TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *
             began = start ? busy : ta;
             tx_len = f.len;
             busy = began + tx_len * (int)PS_PER_BYTE;
+            early += busy < SLOT;
             f.ts = S0 + busy + PROP_PS;
             to = &msg[n_out++];
             if (start)
@@ -350,7 +341,7 @@ TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *
         }
         frame_copy(to, &f); // (write-through: a link's reader loads it from L2)
     }
-    tag_store(&s.msg_tag[msg_index(s, x.gt, out_link)], x.gt << 16 | n_out);
+    msg_seal(s, x.gt, out_link, n_out, early);
     pr.q_head = head;
     pr.q_size = size;
     if (n_out)
@@ -377,28 +368,11 @@ TB_D Input input_of(const SwCtx &x, const SwShared &sh, int q)
     return in;
 }
 
-// phase 1 (lane q < k): clear its row; the window (frames of msg[t-2] from S0 on, of msg[t-1] before E0)
-TB_D int sw_phase_window(const SwCtx &x, SwShared &sh, int q)
+// phase 1 (lane q < k): clear its row
+TB_D void sw_phase_clear(const SwCtx &x, SwShared &sh, int q)
 {
     for (int i = 0; i <= x.sr->k; i++)
         sh.rows()[q][i] = 0;
-    const int64_t S0 = x.t * SLOT_PS, E0 = S0 + SLOT_PS;
-    const int r2 = sh.raw2[q], r1 = sh.raw1[q];
-    // index msg[t-2] (window i2 = 0, n2 = r2, n1 = 0), then msg[t-1] (n2 = 0)
-    sh.win[q][0] = 0;
-    sh.win[q][1] = r2;
-    sh.win[q][2] = 0;
-    Input all = input_of(x, sh, q);
-    int i2 = 0;
-    while (i2 < r2 && all.ts(i2) < S0)
-        i2++;
-    all.n2 = 0;
-    int n1 = 0;
-    while (n1 < r1 && all.ts(n1) < E0)
-        n1++;
-    sh.win[q][0] = i2;
-    sh.win[q][2] = n1;
-    return (r2 - i2) + n1;
 }
 
 TB_D int sw_egress_of(const SwCtx &x, const Input &in, int q, int j)
@@ -557,7 +531,7 @@ TB_D bool sw_phase_egress(const SwCtx &x, SwShared &sh, int e, SwCounts &cn)
         eg.enqueue(p, p.ts);
     }
     eg.advance(eg.horizon - 1);
-    tag_store(&s.msg_tag[msg_index(s, x.gt, out_link)], (int64_t)x.gt << 16 | eg.n_out);
+    msg_seal(s, x.gt, out_link, eg.n_out, eg.early);
     pr.q_head = eg.head;
     pr.q_size = eg.size;
     pr.link_free = eg.busy_until;

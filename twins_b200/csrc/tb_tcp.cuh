@@ -180,30 +180,27 @@ TB_DN void nic_run(HostNic *nic, Frame *list, int n, int until)
 TB_D void to_device(HostCtx &c, int f, uint8_t flags, uint32_t num, uint16_t wire_len, bool toward_sender, uint32_t up, int dst,
                     int64_t now)
 {
-    Frame fr;
+    if (c.list && c.out_n == OUT_FRAMES)
+    {
+        // (a full list: the NIC takes it now; what it starts later in the slot it starts the same)
+        nic_run(c.nic, c.out, c.out_n, (int)(now - c.nic->S0));
+        c.out_n = 0;
+    }
+    Frame own, &fr = c.list ? c.out[c.out_n++] : own;
     fr.ts = now;
     fr.flow = (uint32_t)f;
     fr.sa = num;
     fr.len = wire_len;
     fr.dst = (uint16_t)dst;
     fr.flags = (uint8_t)(flags | (c.dctcp ? F_ECT : 0));
-    fr.to_sender = toward_sender ? 1 : 0;
+    fr.to_sender = (uint8_t)((toward_sender ? 1 : 0) | (c.list && c.kicked == now ? OFFER_KICK : 0));
     fr.up = (uint16_t)up;
     fr.ch = c.ech;
     if (!c.list)
     {
         c.eg.kicked = c.kicked;
         c.eg.enqueue(fr, now);
-        return;
     }
-    if (c.out_n == OUT_FRAMES)
-    {
-        // (a full list: the NIC takes it now; what it starts later in the slot it starts the same)
-        nic_run(c.nic, c.out, c.out_n, (int)(now - c.nic->S0));
-        c.out_n = 0;
-    }
-    fr.to_sender |= c.kicked == now ? OFFER_KICK : 0;
-    frame_copy(&c.out[c.out_n++], &fr);
 }
 TB_D void emit_snd(HostCtx &c, int f, const SndCore &S, uint8_t flags, uint32_t num, uint16_t wire_len, int64_t now)
 {
