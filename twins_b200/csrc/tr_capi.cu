@@ -16,35 +16,63 @@ namespace tr
 
 namespace
 {
-// the run's arrays that start as set-up images, the ones that start zeroed, and the tail ring
+// The run's arrays that start as set-up images, the ones that start zeroed, and the tail ring. A run
+// takes them in one order and of one size (but for a tail ring that grew), so the next run of the
+// batch fills the same memory again: allocating and freeing some forty arrays, gigabytes in all, took
+// 10 ms of a small run and up to 100 ms when the driver was slow about it.
 struct DevArrays
 {
-    std::vector<void *> mem;
-    size_t bytes = 0;
+    struct Piece
+    {
+        void *p;
+        size_t bytes;
+    };
+    std::vector<Piece> mem;
+    size_t at = 0, bytes = 0; // the next piece; the bytes taken by this run
+    cudaStream_t stream = nullptr;
     ~DevArrays() { release(); }
     void release()
     {
-        for (void *p : mem)
-            cudaFree(p);
+        for (Piece &m : mem)
+            cudaFree(m.p);
         mem.clear();
-        bytes = 0;
+        at = bytes = 0;
+    }
+    void begin(cudaStream_t s)
+    {
+        stream = s;
+        at = bytes = 0;
+    }
+    template <class T>
+    bool take(T **p, size_t n)
+    {
+        const size_t b = sizeof(T) * (n ? n : 1);
+        if (at == mem.size())
+            mem.push_back({nullptr, 0});
+        Piece &m = mem[at++];
+        if (m.bytes != b)
+        {
+            cudaFree(m.p);
+            m = {nullptr, 0};
+            if (cudaMalloc(&m.p, b) != cudaSuccess)
+                return false;
+            m.bytes = b;
+        }
+        *p = (T *)m.p;
+        bytes += b;
+        return true;
     }
     template <class T>
     bool zeroed(T **p, size_t n)
     {
-        const size_t b = sizeof(T) * (n ? n : 1);
-        if (cudaMalloc((void **)p, b) != cudaSuccess)
-            return false;
-        mem.push_back(*p);
-        bytes += b;
-        return cudaMemset(*p, 0, b) == cudaSuccess;
+        return take(p, n) && cudaMemsetAsync(*p, 0, sizeof(T) * (n ? n : 1), stream) == cudaSuccess;
     }
     template <class T>
     bool copy(T **p, const std::vector<T> &v)
     {
-        if (!zeroed(p, v.size()))
-            return false;
-        return v.empty() || cudaMemcpy(*p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+        if (v.empty())
+            return zeroed(p, 0);
+        return take(p, v.size()) && cudaMemcpyAsync(*p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream) == cudaSuccess;
     }
 };
 } // namespace
@@ -85,7 +113,7 @@ struct RdmaRun
     // the initial state on the device: set-up images copied, the rest zeroed
     bool upload(std::string *err)
     {
-        d.release();
+        d.begin(stream);
         const RLayout &l = L;
         RSim x{};
         x.H = l.H, x.S = l.S, x.F = l.F, x.W = l.W, x.P = l.P;
@@ -124,9 +152,9 @@ struct RdmaRun
         x.tx_cap = tx_cap;
         x.tx_from = tx_from;
         x.tx_until = tx_until;
-        // (the zeroing and copies above run on the legacy default stream, which the run's own
-        // non-blocking stream does not wait for: all of it must be done before the first launch)
-        if (cudaDeviceSynchronize() != cudaSuccess)
+        // (the zeroing and copies above run on the run's own stream, before its first launch; the copies'
+        // sources are this function's)
+        if (cudaStreamSynchronize(stream) != cudaSuccess)
         {
             *err = std::string("device memory for the RDMA run: ") + cudaGetErrorString(cudaGetLastError());
             d.release();
