@@ -92,6 +92,7 @@ struct RdmaRun
     unsigned long long tx_total = 0;
     int grid = 0;
     size_t smem = 0;
+    const void *kernel = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     std::vector<int64_t> fct;
@@ -216,7 +217,7 @@ int rdma_prepare(RdmaRun *r, std::string *err)
         cudaEventCreate(&r->e0);
         cudaEventCreate(&r->e1);
     }
-    if (int e = rdma_launch_shape(r->L.max_deg, (r->L.H + RDMA_WARPS - 1) / RDMA_WARPS + r->L.S, &r->grid, &r->smem))
+    if (int e = rdma_launch_shape(r->L.max_deg, (r->L.H + RDMA_WARPS - 1) / RDMA_WARPS + r->L.S, &r->grid, &r->smem, &r->kernel))
         return *err = std::string("the RDMA slot kernel does not fit: ") + cudaGetErrorString((cudaError_t)e), -2;
     r->prepared = true;
     return 0;
@@ -250,7 +251,7 @@ int rdma_run(RdmaRun *r, long long max_slots, std::string *err)
         {
             cudaEventRecord(r->e0, r->stream);
             const int slots = 4096;
-            if (int e = rdma_launch(s, r->grid, r->smem, slots, r->L.max_deg, r->stream))
+            if (int e = rdma_launch(s, r->kernel, r->grid, r->smem, slots, r->L.max_deg, r->stream))
                 return *err = std::string("RDMA slot kernel launch: ") + cudaGetErrorString((cudaError_t)e), -2;
             cudaEventRecord(r->e1, r->stream);
             if (cudaMemcpyAsync(&ctl, s.ctl, sizeof ctl, cudaMemcpyDeviceToHost, r->stream) != cudaSuccess ||

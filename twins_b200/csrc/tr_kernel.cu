@@ -46,8 +46,10 @@ __host__ __device__ inline size_t block_scratch_bytes(int max_deg)
 }
 
 // A block's units: a group of RDMA_WARPS NIC hosts (a warp each) or one switch (all its warps: its
-// egress ports spread over them in safe slots).
-__global__ void __launch_bounds__(RDMA_WARPS * 32) rdma_slot_kernel(RSim s, int slots, int max_deg)
+// egress ports spread over them in safe slots). MIN_BLOCKS: the register budget, chosen per launch
+// (rdma_launch_shape). The parameters stay in the constant bank (their address is taken).
+template <int MIN_BLOCKS>
+__global__ void __launch_bounds__(RDMA_WARPS * 32, MIN_BLOCKS) rdma_slot_kernel(const __grid_constant__ RSim s, int slots, int max_deg)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int blk_last;
@@ -154,15 +156,24 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32) rdma_slot_kernel(RSim s, int 
     }
 }
 
-int rdma_launch_shape(int max_deg, int units, int *grid, size_t *smem)
+// The kernel of `units` units: with 168 registers (3 blocks per SM), unless 128 (4 blocks, spilling) let
+// every unit have a resident block of its own and 168 do not. Measured, 3 / 4 blocks: FatTree k=16
+// (576 units) 91 / 85 ms; eight k=8 worlds (896 units) 279 / 293 ms.
+static const void *rdma_kernel_of(int units, int sms)
+{
+    return units > 3 * sms && units <= 4 * sms ? (const void *)rdma_slot_kernel<4> : (const void *)rdma_slot_kernel<3>;
+}
+
+int rdma_launch_shape(int max_deg, int units, int *grid, size_t *smem, const void **kernel)
 {
     *smem = block_scratch_bytes(max_deg);
-    if (cudaFuncSetAttribute((const void *)rdma_slot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess)
-        return (int)cudaGetLastError();
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)rdma_slot_kernel, RDMA_WARPS * 32, *smem) != cudaSuccess)
+    *kernel = rdma_kernel_of(units, sms);
+    if (cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess)
+        return (int)cudaGetLastError();
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, *kernel, RDMA_WARPS * 32, *smem) != cudaSuccess)
         return (int)cudaGetLastError();
     if (per_sm < 1)
         return (int)cudaErrorInvalidConfiguration;
@@ -172,10 +183,10 @@ int rdma_launch_shape(int max_deg, int units, int *grid, size_t *smem)
     return 0;
 }
 
-int rdma_launch(const RSim &s, int grid, size_t smem, int slots, int max_deg, cudaStream_t stream)
+int rdma_launch(const RSim &s, const void *kernel, int grid, size_t smem, int slots, int max_deg, cudaStream_t stream)
 {
     void *args[] = {(void *)&s, (void *)&slots, (void *)&max_deg};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)rdma_slot_kernel, dim3(grid), dim3(RDMA_WARPS * 32), args, smem, stream);
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(RDMA_WARPS * 32), args, smem, stream);
     return e == cudaSuccess ? 0 : (int)e;
 }
 

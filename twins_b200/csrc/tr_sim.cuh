@@ -589,12 +589,23 @@ TR_HD int64_t link_tx_ns(const RSim &s, const LinkInfo &l, uint32_t bytes)
     return tx_ns(l.bps, bytes);
 }
 
+// a / b and a % b of numbers at least 0: the 32-bit division where both fit (slot numbers and the
+// first 4 s of times do), a quarter of the 64-bit one's instructions
+TR_HD int64_t quot(int64_t a, int64_t b)
+{
+    return (uint64_t)a >> 32 || (uint64_t)b >> 32 ? a / b : (int64_t)((uint32_t)a / (uint32_t)b);
+}
+TR_HD int64_t rem(int64_t a, int64_t b)
+{
+    return (uint64_t)a >> 32 || (uint64_t)b >> 32 ? a % b : (int64_t)((uint32_t)a % (uint32_t)b);
+}
+
 // a sender's place in its out link's ring: the bucket of the slot its frames arrive in
 struct OutLink
 {
     int link;
     LinkInfo li;
-    int64_t lo, hi;      // the open bucket's times (hi 0: none open)
+    int64_t slot, hi;    // the open bucket's slot and the end of its times (hi 0: none open)
     uint64_t base;       // its first frame in msg
     uint32_t tag_at;     // its tag in msg_cnt
     uint32_t n;          // frames in it
@@ -611,7 +622,7 @@ struct OutLink
     {
         if (hi == 0)
             return;
-        last = (long long)(lo / s.D) << 16 | n;
+        last = (long long)slot << 16 | n;
         s.msg_cnt[tag_at] = last;
         hi = 0;
     }
@@ -621,14 +632,14 @@ struct OutLink
         if (ts >= hi)
         {
             flush(s);
-            const int64_t a = ts / s.D;
-            const int b = (int)(a % li.nb);
+            const int64_t a = quot(ts, s.D);
+            const int b = (int)rem(a, li.nb);
             tag_at = li.coff + (uint32_t)b;
-            lo = a * s.D;
-            hi = lo + s.D;
+            slot = a;
+            hi = (a + 1) * s.D;
             base = li.moff + (uint64_t)b * li.cap;
             n = (last >> 16) == a ? (uint32_t)(last & 0xFFFF) : 0;
-            s.pend[a % s.pend_n] = 1;
+            s.pend[rem(a, s.pend_n)] = 1;
         }
         if (n >= li.cap)
         {
@@ -643,7 +654,7 @@ struct OutLink
 TR_HD int bucket_of(const RSim &s, int link, int64_t t, uint64_t *base)
 {
     const LinkInfo &l = s.link[link];
-    const int b = (int)(t % l.nb);
+    const int b = (int)rem(t, l.nb);
     const long long tag = ld_tag(&s.msg_cnt[l.coff + b]);
     *base = l.moff + (uint64_t)b * l.cap;
     return (tag >> 16) == t ? (int)(tag & 0xFFFF) : 0;
@@ -667,6 +678,7 @@ __device__ __forceinline__ void group_sync(int lanes)
 __device__ __forceinline__ void sh_add(uint32_t *p, uint32_t v) { atomicAdd(p, v); }
 __device__ __forceinline__ void sh_add(int *p, int v) { atomicAdd(p, v); }
 __device__ __forceinline__ void sh_sub(uint32_t *p, uint32_t v) { atomicSub(p, v); }
+__device__ __forceinline__ int sh_take(int *p) { return atomicSub(p, 1) - 1; } // (one less than before)
 __device__ __forceinline__ void ld_pkt(Pkt &p, const Pkt *src)
 {
     const uint4 *s = reinterpret_cast<const uint4 *>(src);
@@ -692,6 +704,7 @@ inline void prefetch_l1(const void *) {}
 inline void sh_add(uint32_t *p, uint32_t v) { *p += v; }
 inline void sh_add(int *p, int v) { *p += v; }
 inline void sh_sub(uint32_t *p, uint32_t v) { *p -= v; }
+inline int sh_take(int *p) { return --*p; }
 inline void ld_pkt(Pkt &p, const Pkt *src) { p = *src; }
 inline void ld_chain(Chain &c, const Chain *src) { c = *src; }
 #endif
@@ -703,7 +716,7 @@ struct SArr
     int64_t ts;
     uint32_t acode;
     uint32_t frame;
-    uint32_t flow;
+    uint32_t flow;    // (a switch's safe slot: the arrival at this place of the ports' orders, safe_order)
     int16_t out;      // egress port (-1: a PFC frame, or no route)
     uint8_t q, in;    // its queue; its ingress port
     uint16_t size;
@@ -1259,7 +1272,7 @@ struct alignas(16) SwPort
     uint64_t abase;        // its arrivals' bucket in msg
     int an, first;         // its arrivals this slot; the first one's place among the staged
     int nout;              // frames it sent this slot
-    int ai, aend;          // the serial path's cursor over its arrivals
+    int ai, aend;          // the serial path's cursor over its arrivals; safe slots: arrivals leaving by it, whether two at one time
     uint32_t ing0, abytes; // safe slots: its ingress bytes at the slot's start; bytes arriving on it for queue PG
     int ocnt, obase;       // safe slots: arrivals leaving by it; their place in the order array
     SArr pa;               // the unstaged serial path's next arrival
@@ -1285,7 +1298,6 @@ struct SwEv
     SwInfo si;
     MmuSwitch mmu;
     SwPort *pe;
-    bool safe; // no buffer decision can occur in this slot: lanes run egress ports apart
     TailChunk *tail; // the tail positions of the running event's port (its lane's alone)
     int64_t now;
     Chain cur;
@@ -1375,34 +1387,29 @@ TR_HD void s_send_pfc(SwEv &e, int port, bool resume)
         s_start_q0(e, port);
 }
 
+// the INT word of a data frame leaving port `pe`, in its hop words (int_stamp; every word is a choice,
+// so that the frame stays in registers)
+TR_HD void s_stamp(const SwEv &e, const SwPort &pe, Pkt &p)
+{
+    if (p.nhop == 0xFFFF)
+        return;
+    const uint64_t word = hop_make((uint64_t)e.now, pe.pt.tx_bytes, pe.pt.bytes_total, pe.info.bps, e.w->cc.int_multi);
+    const int at = p.nhop % MAX_HOP;
+    for (int k = 0; k < MAX_HOP; k++)
+        p.hop[k] = k == at ? word : p.hop[k];
+    p.nhop++;
+}
+
 // a frame of queue PG leaves: the buffer gives its bytes back, ECN may mark it, a paused ingress
-// may resume, an HPCC data frame takes the port's INT word; then TransmitStart. In a safe slot only
-// the ingress and egress byte counts change (no headroom is in use and no port is paused).
+// may resume, an HPCC data frame takes the port's INT word; then TransmitStart
 TR_HD void s_start_q3(SwEv &e, int port, Pkt p)
 {
     const RWorld &w = *e.w;
     SwPort &pe = e.pe[port];
     SwPort &in = e.pe[p.inport];
     tb::Rng &rng = pe.pt.rng;
-    unsigned r;
-    if (e.safe)
-    {
-        sh_sub(&in.pt.mmu.ing, p.size);
-        pe.pt.mmu.egr -= p.size;
-        r = 0;
-        if (w.ecn)
-        {
-            const uint32_t egr = pe.pt.mmu.egr;
-            if (egr > pe.info.kmax)
-                r = MMU_MARK;
-            else if (egr > pe.info.kmin &&
-                     tb::rand_u01(rng) < pe.info.pmax * (double)(egr - pe.info.kmin) / (double)(pe.info.kmax - pe.info.kmin))
-                r = MMU_MARK;
-        }
-    }
-    else
-        r = mmu_release(w.buffer_size, e.mmu, in.pt.mmu, in.info.shift, pe.pt.mmu, p.size, w.ecn != 0, pe.info.kmin, pe.info.kmax,
-                        pe.info.pmax, false, [&]() { return tb::rand_u01(rng); });
+    const unsigned r = mmu_release(w.buffer_size, e.mmu, in.pt.mmu, in.info.shift, pe.pt.mmu, p.size, w.ecn != 0, pe.info.kmin, pe.info.kmax,
+                                   pe.info.pmax, false, [&]() { return tb::rand_u01(rng); });
     if (r & MMU_MARK)
     {
         p.ecn = 3;
@@ -1411,7 +1418,7 @@ TR_HD void s_start_q3(SwEv &e, int port, Pkt p)
     if (r & MMU_RESUME)
         s_send_pfc(e, p.inport, true);
     if (p.kind == K_DATA && w.nic.cc == 3)
-        int_stamp(p.hop, p.nhop, e.now, pe.pt.tx_bytes, pe.pt.bytes_total, pe.info.bps, w.cc.int_multi);
+        s_stamp(e, pe, p);
     pe.pt.tx_bytes += p.size;
     s_transmit(e, port, p);
 }
@@ -1457,24 +1464,15 @@ TR_HD void s_forward(SwEv &e, int inport, Pkt p, int out, int q)
         return;
     if (q != 0)
     {
-        if (e.safe)
+        SwPort &in = e.pe[inport];
+        const unsigned r = mmu_admit(e.w->buffer_size, e.mmu, in.pt.mmu, in.info.hdrm_cap, in.info.shift, e.pe[out].pt.mmu, p.size, false);
+        if (r & MMU_DROP)
         {
-            // below every threshold for the whole slot: no drop, no headroom, no PAUSE
-            sh_add(&e.pe[inport].pt.mmu.ing, (uint32_t)p.size);
-            e.pe[out].pt.mmu.egr += p.size;
+            count(*e.s, EV_DROP);
+            return;
         }
-        else
-        {
-            SwPort &in = e.pe[inport];
-            const unsigned r = mmu_admit(e.w->buffer_size, e.mmu, in.pt.mmu, in.info.hdrm_cap, in.info.shift, e.pe[out].pt.mmu, p.size, false);
-            if (r & MMU_DROP)
-            {
-                count(*e.s, EV_DROP);
-                return;
-            }
-            if (r & MMU_PAUSE)
-                s_send_pfc(e, inport, false);
-        }
+        if (r & MMU_PAUSE)
+            s_send_pfc(e, inport, false);
     }
     p.inport = (uint8_t)inport;
     Port &o = e.pe[out].pt;
@@ -1507,8 +1505,7 @@ TR_HD void arr_pkt(const RSim &s, const SwWork &w, const SArr &a, Pkt &p)
 TR_HD void s_arrival(SwEv &e, const SwWork &w, const SArr &a)
 {
     const RSim &s = *e.s;
-    if (!e.safe)
-        e.tail = &e.pe[a.in].pt.tail;
+    e.tail = &e.pe[a.in].pt.tail;
     Chain c;
     arr_chain(s, w, a, c);
     chain_push(s, e.cur, a.acode, c, *e.tail);
@@ -1541,8 +1538,7 @@ TR_HD void s_arrival(SwEv &e, const SwWork &w, const SArr &a)
 // a port's TransmitComplete
 TR_HD void s_tc(SwEv &e, int port)
 {
-    if (!e.safe)
-        e.tail = &e.pe[port].pt.tail;
+    e.tail = &e.pe[port].pt.tail;
     e.cur = e.pe[port].tc;
     e.ord = 0;
     e.n_ev++;
@@ -1569,35 +1565,91 @@ TR_HD bool arr_before_tc(const RSim &s, const SwWork &w, const SArr &a, const Ch
     return runs_before(s, a.ts, a.acode, ca, a.ts, 0, tc);
 }
 
+// the port whose events a staged arrival is among in a safe slot: its egress, or its own for a PFC frame
+TR_HD int own_port(const SArr &a) { return a.out >= 0 ? a.out : (a.kind == K_PAUSE || a.kind == K_RESUME ? a.in : -1); }
+
+// A safe slot's arrivals in each egress port's order, by the group's lanes, an arrival per lane: its
+// place is the number of its port's arrivals before it (by time, then as staged); the order of port
+// o is arr[obase + i].flow, i < ai. Ports with two arrivals at one time (aend) order those by their
+// chains on their own lane (safe_ties). (An insertion by the port's lane, scanning every staged
+// arrival, took 40% of a safe slot: 512 slots of HPCC k=16, 20 us each.)
+TR_HD void safe_order(const SwWork &w, int deg, int total, int lane, int lanes)
+{
+    for (int p = lane; p < deg; p += lanes)
+    {
+        w.port[p].ai = w.port[p].ocnt;
+        w.port[p].aend = 0;
+    }
+    group_sync(lanes);
+    for (int j = lane; j < total; j += lanes)
+    {
+        const int o = own_port(w.arr[j]);
+        if (o >= 0)
+            w.ord[w.port[o].obase + sh_take(&w.port[o].ocnt)] = (uint16_t)j;
+    }
+    group_sync(lanes);
+    for (int j = lane; j < total; j += lanes)
+    {
+        const int o = own_port(w.arr[j]);
+        if (o < 0)
+            continue;
+        const uint16_t *mine = w.ord + w.port[o].obase;
+        const int n = w.port[o].ai;
+        const int64_t ts = w.arr[j].ts;
+        int rank = 0, same = 0;
+        for (int i = 0; i < n; i++)
+        {
+            const int k = mine[i];
+            const int64_t t = w.arr[k].ts;
+            rank += t < ts || (t == ts && k < j);
+            same += t == ts;
+        }
+        w.arr[w.port[o].obase + rank].flow = (uint32_t)j;
+        if (same > 1)
+            w.port[o].aend = 1;
+    }
+    group_sync(lanes);
+}
+
+// port o's arrivals at one time, in event order (insertion as staged; an undecided tie keeps the
+// earlier port's arrival first)
+TR_HD void safe_ties(const RSim &s, const SwWork &w, int o)
+{
+    SArr *list = w.arr + w.port[o].obase;
+    for (int i = 1; i < w.port[o].ai; i++)
+    {
+        const uint32_t j = list[i].flow;
+        int k = i;
+        for (; k > 0 && w.arr[list[k - 1].flow].ts == w.arr[j].ts && arr_before(s, w, w.arr[j], w.arr[list[k - 1].flow]); k--)
+            list[k].flow = list[k - 1].flow;
+        list[k].flow = j;
+    }
+}
+
 // A safe slot's egress port o, on its own lane: the arrivals routed to it (and PFC frames arriving
 // at it) in event order, merged with its TransmitCompletes. Restricting ns-3's order to one port's
-// events keeps their order, and in a safe slot ports meet only in their ingress byte counts.
-TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1, int total)
+// events keeps their order, and in a safe slot ports meet only in their ingress byte counts. An
+// iteration is an event of either kind: its chain, then the frame it starts (the arrival itself
+// at an idle port, or the queue's next) or queues, in one piece of code, so that the lanes of a warp
+// take their events together. (With a function per kind of event, each with the transmission inside,
+// the lanes ran one after another.)
+TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1)
 {
     const RSim &s = *e.s;
+    const RWorld &rw = *e.w;
     SwPort &me = e.pe[o];
-    e.tail = &me.pt.tail;
-    uint16_t *list = w.ord + me.obase; // (this port's share of the order array)
-    int n = 0;
-    for (int j = 0; j < total; j++)
-    {
-        const SArr &a = w.arr[j];
-        const int own = a.out >= 0 ? a.out : (a.kind == K_PAUSE || a.kind == K_RESUME ? a.in : -1);
-        if (own != o)
-            continue;
-        // insertion in event order (an undecided tie keeps the earlier port's arrival first)
-        int k = n++;
-        while (k > 0 && arr_before(s, w, a, w.arr[list[k - 1]]))
-        {
-            list[k] = list[k - 1];
-            k--;
-        }
-        list[k] = (uint16_t)j;
-    }
+    Port &pt = me.pt;
+    const size_t pi = (size_t)e.si.pbase + o;
+    e.tail = &pt.tail;
+    if (me.aend)
+        safe_ties(s, w, o);
+    const SArr *list = w.arr + me.obase; // (this port's share of the order)
+    const int n = me.ai;
     int i = 0;
     for (;;)
     {
-        const int64_t ta = i < n ? w.arr[list[i]].ts : INT64_MAX, tc = me.pt.tc_at;
+        const SArr &a = w.arr[i < n ? list[i].flow : 0];
+        const int64_t ta = i < n ? a.ts : INT64_MAX, tc = pt.tc_at;
         const bool htc = tc >= 0 && tc < t1;
         if (ta == INT64_MAX && !htc)
             break;
@@ -1607,16 +1659,92 @@ TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1, int total)
         else if (ta != tc)
             arr = ta < tc;
         else
-            arr = arr_before_tc(s, w, w.arr[list[i]], me.tc);
-        if (!arr)
+            arr = arr_before_tc(s, w, a, me.tc);
+        i += arr;
+        e.now = arr ? ta : tc;
+        e.n_ev++;
+        e.n_arr += arr;
+        e.ord = 0;
+        // the event's chain
+        if (arr && a.copy == NO_COPY)
+            ld_chain(e.cur, &s.msg[a.frame].c);
+        else
+            e.cur = arr ? w.fr[a.copy].c : me.tc;
+        if (arr)
+            chain_push(s, e.cur, a.acode, e.cur, *e.tail);
+        else
+            pt.tc_at = -1;
+        // what it does: a frame of its own to start or to queue, or the queues' next
+        const bool pfc = arr && (a.kind == K_PAUSE || a.kind == K_RESUME), frame = arr && !pfc;
+        Pkt p;
+        bool start = false, counted = false, next = !arr; // (counted: a frame of queue PG, in the buffer's counts)
+        if (arr)
         {
-            e.now = tc;
-            s_tc(e, o);
-            continue;
+            if (a.copy == NO_COPY)
+                ld_pkt(p, &s.msg[a.frame].p);
+            else
+                p = w.fr[a.copy].p;
         }
-        const SArr &a = w.arr[list[i++]];
-        e.now = a.ts;
-        s_arrival(e, w, a);
+        if (pfc && rw.qbb)
+        {
+            pt.paused = a.kind == K_PAUSE ? pt.paused | 1u << p.q : pt.paused & ~(1u << p.q);
+            next = a.kind == K_RESUME;
+        }
+        if (frame)
+        {
+            p.inport = a.in;
+            if (a.q != 0)
+            {
+                // below every threshold for the whole slot: no drop, no headroom, no PAUSE
+                sh_add(&e.pe[a.in].pt.mmu.ing, (uint32_t)p.size);
+                pt.mmu.egr += p.size;
+            }
+            start = counted = a.q != 0 && pt.tc_at < 0 && pt.q0_n == 0 && pt.q3_n == 0 && !(pt.paused >> PG & 1);
+            if (!start)
+            {
+                s_enqueue(e, o, a.q, p);
+                next = true;
+            }
+        }
+        if (next && pt.tc_at < 0)
+        {
+            if (pt.q0_n > 0)
+            {
+                // (queue 0's frames pass no buffer accounting)
+                p = s.q0[pi * s.q0_cap + pt.q0_head];
+                pt.q0_head = pt.q0_head + 1 == s.q0_cap ? 0 : pt.q0_head + 1;
+                pt.q0_n--;
+                start = true;
+            }
+            else if (!(pt.paused >> PG & 1) && pt.q3_n > 0)
+            {
+                p = s.q3[pi * s.q3_cap + pt.q3_head];
+                pt.q3_head = pt.q3_head + 1 == s.q3_cap ? 0 : pt.q3_head + 1;
+                pt.q3_n--;
+                start = counted = true;
+            }
+            if (start)
+                pt.bytes_total -= p.size;
+        }
+        if (!start)
+            continue;
+        if (counted)
+        {
+            sh_sub(&e.pe[p.inport].pt.mmu.ing, p.size);
+            pt.mmu.egr -= p.size;
+            const uint32_t egr = pt.mmu.egr;
+            if (rw.ecn && (egr > me.info.kmax ||
+                           (egr > me.info.kmin &&
+                            tb::rand_u01(pt.rng) < me.info.pmax * (double)(egr - me.info.kmin) / (double)(me.info.kmax - me.info.kmin))))
+            {
+                p.ecn = 3;
+                count(s, EV_MARK);
+            }
+            if (p.kind == K_DATA && rw.nic.cc == 3)
+                s_stamp(e, me, p);
+        }
+        pt.tx_bytes += p.size;
+        s_transmit(e, o, p);
     }
 }
 
@@ -1887,7 +2015,6 @@ TR_HD bool switch_slot(const RSim &s, int x, int64_t t, const SwWork &w, int lan
     }
     group_sync(lanes);
     const bool safe = w.flags[2] != 0;
-    e.safe = safe;
     SW_PHASE(2);
 #ifdef TR_PROFILE
     if (lane == 0)
@@ -1895,10 +2022,11 @@ TR_HD bool switch_slot(const RSim &s, int x, int64_t t, const SwWork &w, int lan
 #endif
     if (safe)
     {
-        // egress ports spread over the warps (a warp's lanes diverge: fewer ports each, less waiting)
+        safe_order(w, deg, total, lane, lanes);
+        // egress ports spread over the warps
         const int wl = lanes < 32 ? lanes : 32, nw = lanes < 32 ? 1 : lanes / 32;
         for (int o = lane / wl + nw * (lane % wl); o < deg; o += nw * wl)
-            safe_egress(e, w, o, t1, total);
+            safe_egress(e, w, o, t1);
 #if defined(TR_PROFILE) && defined(__CUDA_ARCH__)
         atomicMax(&s.ev[EV_PROF_LANE_EV_SLOT], e.n_ev);
 #endif
