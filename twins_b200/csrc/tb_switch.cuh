@@ -233,9 +233,11 @@ struct SwCounts
 // do. Times are offsets in the slot. A queued frame always begins when the wire gets free: it was
 // queued because the wire was busy beyond its arrival (an arrival at an idle wire starts at once,
 // which is when Egress's next step would start it), so its chain is the child of the wire's
-// frame's. Bound by the latency of a frame's load and chain, about 1 us per iteration; the frames queued
-// next are in L1 (sw_prefetch). Returns true if the port sent or holds frames.
-TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *list, int n, SwCounts &c)
+// frame's. A frame that joins the queue stays where it is staged, and goes to the queue's ring in
+// memory if it still waits when the slot ends: read back from the ring it would wait for its own store
+// (600 cycles). Bound by the latency of a frame's load and chain, well under 1 us per iteration; the
+// ring's first frames are in L1. Returns true if the port sent or holds frames.
+TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, uint32_t *list, int n, SwCounts &c)
 {
     const Sim &s = *x.s;
     constexpr int SLOT = (int)SLOT_PS;
@@ -261,16 +263,19 @@ TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *
         began = busy - tx_len * (int)PS_PER_BYTE;
     }
     Chain wire = pr.last;
-    int i = 0;
+    // queued: `held` frames of the ring, then lq from list[jq] on (~0: dropped)
+    int i = 0, held = size, jq = 0, lq = 0;
     uint32_t next = n > 0 ? list[0] : 0;
     for (;;)
     {
         const int ta = i < n ? (int)(next >> 9) : SLOT;
+        size = held + lq;
         const bool start = size > 0 && busy < SLOT && busy <= ta;
         if (!start && i >= n)
             break;
         Frame f;
-        frame_copy(&f, start ? &ring[head] : &sh.fr()[next & 511]);
+        Frame *const here = &sh.fr()[(start ? list[jq] : next) & 511];
+        frame_copy(&f, start && held ? &ring[head] : here);
         const bool idle = size == 0 && busy <= ta; // (an arrival at an idle wire)
         bool sends = start || idle, gone = false;
         if (sends && n_out == MAX_TX)
@@ -291,8 +296,6 @@ TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *
         {
             const int backlog = !size || busy <= ta ? size : size - (began < ta ? 1 : 0);
             f.ts = S0 + ta;
-            i++;
-            next = i < n ? list[i] : 0;
             if (backlog >= red_k && backlog > 1)
             {
                 if (f.flags & F_ECT)
@@ -314,10 +317,16 @@ TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *
                 c.ovf++;
                 gone = true;
             }
+            if (gone)
+                list[i] = ~0u;
+            if (lq == 0)
+                jq = gone || sends ? i + 1 : i;
+            lq += !gone && !sends;
+            i++;
+            next = i < n ? list[i] : 0;
         }
         if (gone)
             continue;
-        Frame *to;
         if (sends)
         {
             wire = f.ch;
@@ -326,21 +335,33 @@ TB_D bool sw_egress_staged(const SwCtx &x, SwShared &sh, int e, const uint32_t *
             busy = began + tx_len * (int)PS_PER_BYTE;
             early += busy < SLOT;
             f.ts = S0 + busy + PROP_PS;
-            to = &msg[n_out++];
-            if (start)
+            frame_store_link(&msg[n_out++], f);
+            if (start && held)
             {
                 head = head + 1 == cap ? 0 : head + 1;
-                size--;
+                held--;
+            }
+            else if (start)
+            {
+                lq--;
+                jq++;
+                while (jq < i && list[jq] == ~0u)
+                    jq++;
             }
         }
         else
-        {
-            const int at = head + size;
-            to = &ring[at < cap ? at : at - cap];
-            size++;
-        }
-        frame_copy(to, &f); // (write-through: a link's reader loads it from L2)
+            frame_copy(here, &f);
     }
+    for (; lq; jq++)
+    {
+        if (list[jq] == ~0u)
+            continue;
+        const int at = head + held;
+        frame_copy(&ring[at < cap ? at : at - cap], &sh.fr()[list[jq] & 511]);
+        held++;
+        lq--;
+    }
+    size = held;
     msg_seal(s, x.gt, out_link, n_out, early);
     pr.q_head = head;
     pr.q_size = size;
