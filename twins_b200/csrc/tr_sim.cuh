@@ -1632,7 +1632,8 @@ TR_HD void safe_ties(const RSim &s, const SwWork &w, int o)
 // iteration is an event of either kind: its chain, then the frame it starts (the arrival itself
 // at an idle port, or the queue's next) or queues, in one piece of code, so that the lanes of a warp
 // take their events together. (With a function per kind of event, each with the transmission inside,
-// the lanes ran one after another.)
+// the lanes ran one after another.) A frame queued in the slot stays where it was staged until it
+// starts or the slot ends: read back from the queue's ring it would wait for its own store.
 TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1)
 {
     const RSim &s = *e.s;
@@ -1645,6 +1646,11 @@ TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1)
         safe_ties(s, w, o);
     const SArr *list = w.arr + me.obase; // (this port's share of the order)
     const int n = me.ai;
+    int held = pt.q3_n, jq = 0; // queue PG: the frames in its ring, then those queued from list[jq] on (marked pre)
+    auto staged_pkt = [&](const SArr &a, Pkt &p) {
+        arr_pkt(s, w, a, p);
+        p.inport = a.in;
+    };
     int i = 0;
     for (;;)
     {
@@ -1700,11 +1706,17 @@ TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1)
                 pt.mmu.egr += p.size;
             }
             start = counted = a.q != 0 && pt.tc_at < 0 && pt.q0_n == 0 && pt.q3_n == 0 && !(pt.paused >> PG & 1);
-            if (!start)
+            if (!start && a.q == 0)
+                s_enqueue(e, o, 0, p);
+            else if (!start && pt.q3_n >= s.q3_cap)
+                count(s, EV_OVF_QUEUE);
+            else if (!start)
             {
-                s_enqueue(e, o, a.q, p);
-                next = true;
+                w.arr[list[i - 1].flow].pre = 1;
+                pt.q3_n++;
+                pt.bytes_total += p.size;
             }
+            next = !start;
         }
         if (next && pt.tc_at < 0)
         {
@@ -1718,8 +1730,18 @@ TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1)
             }
             else if (!(pt.paused >> PG & 1) && pt.q3_n > 0)
             {
-                p = s.q3[pi * s.q3_cap + pt.q3_head];
-                pt.q3_head = pt.q3_head + 1 == s.q3_cap ? 0 : pt.q3_head + 1;
+                if (held > 0)
+                {
+                    p = s.q3[pi * s.q3_cap + pt.q3_head];
+                    pt.q3_head = pt.q3_head + 1 == s.q3_cap ? 0 : pt.q3_head + 1;
+                    held--;
+                }
+                else
+                {
+                    while (!w.arr[list[jq].flow].pre)
+                        jq++;
+                    staged_pkt(w.arr[list[jq++].flow], p);
+                }
                 pt.q3_n--;
                 start = counted = true;
             }
@@ -1745,6 +1767,19 @@ TR_HD void safe_egress(SwEv &e, const SwWork &w, int o, int64_t t1)
         }
         pt.tx_bytes += p.size;
         s_transmit(e, o, p);
+    }
+    // what waits goes to the ring
+    for (; held < pt.q3_n; jq++)
+    {
+        const SArr &a = w.arr[list[jq].flow];
+        if (!a.pre)
+            continue;
+        Pkt p;
+        staged_pkt(a, p);
+        int at = pt.q3_head + held++;
+        if (at >= s.q3_cap)
+            at -= s.q3_cap;
+        s.q3[pi * s.q3_cap + at] = p;
     }
 }
 
