@@ -286,11 +286,12 @@ struct SentList
     TB_D uint32_t beg(uint32_t i) const { return start[pos(i)]; }
     TB_D uint32_t end(uint32_t i) const { return i + 1 < S.it_n ? start[pos(i + 1)] : S.high; }
     TB_D static uint32_t spread(uint8_t f) { return (f & 1u) | (f & 2u) << 7 | (f & 4u) << 14; } // (flag bits -> plane bits)
-    TB_D uint8_t flags_at(uint32_t p) const
+    TB_D static uint8_t flags_in(uint32_t word, uint32_t p)
     {
-        const uint32_t w = word(p >> 3) >> (p & 7);
+        const uint32_t w = word >> (p & 7);
         return (uint8_t)((w & 1u) | (w >> 7 & 2u) | (w >> 14 & 4u));
     }
+    TB_D uint8_t flags_at(uint32_t p) const { return flags_in(word(p >> 3), p); }
     TB_D void write_at(uint32_t p, uint8_t f)
     {
         const uint32_t b = p & 7;
@@ -526,13 +527,21 @@ TB_D uint32_t ack_drop(SentList &L, uint32_t ack)
     // (the walk keeps the head, the count and the flags' byte sums in registers and settles the
     // record once; an item leaving keeps its stale flag bits, which no read reaches)
     const uint32_t n = S.it_n, high = S.high;
+    // (an item's end and the flags' word are read an item ahead)
     uint32_t head = S.it_head, left = 0, gone = 0, sack = 0, lost = 0, retx = 0, cand = 0, nsack = 0;
-    uint32_t b = n ? L.start[head] : 0;
+    uint32_t nx = head + 1 == L.cap ? 0 : head + 1, wi = head >> 3;
+    uint32_t b = n ? L.start[head] : 0, after = n ? L.start[nx] : 0, w = n ? L.word(wi) : 0;
     while (left < n)
     {
-        const uint32_t nx = head + 1 == L.cap ? 0 : head + 1;
-        const uint32_t e = left + 1 < n ? L.start[nx] : high;
-        const uint8_t f = L.flags_at(head);
+        const uint32_t e = left + 1 < n ? after : high;
+        const uint32_t nx2 = nx + 1 == L.cap ? 0 : nx + 1;
+        after = L.start[nx2];
+        if (head >> 3 != wi)
+        {
+            wi = head >> 3;
+            w = L.word(wi);
+        }
+        const uint8_t f = SentList::flags_in(w, head);
         const uint32_t len = ack < e ? (ack > b ? ack - b : 0) : e - b; // (whole, or the acknowledged part)
         sack += (f & FL_SACK) ? len : 0;
         lost += (f & FL_LOST) ? len : 0;
@@ -548,6 +557,7 @@ TB_D uint32_t ack_drop(SentList &L, uint32_t ack)
         gone += len;
         left++;
         head = nx;
+        nx = nx2;
         b = e;
     }
     S.sack_b -= sack;
@@ -760,9 +770,17 @@ struct RttLog
     {
         if (!S.h_n)
             return;
+        // (the first three entries' ends at once: an ACK mostly covers two)
         const uint32_t k = slot(0);
-        if (at[k] >= 0 && ack >= hi[k])
-            rtt_update(S, now - at[k]);
+        const uint32_t h0 = hi[k], h1 = hi[slot(1)], h2 = hi[slot(2)];
+        const int64_t t = at[k];
+        if (t >= 0 && ack >= h0)
+            rtt_update(S, now - t);
+        const uint32_t n = h0 > ack ? 0 : S.h_n == 1 || h1 > ack ? 1 : S.h_n == 2 || h2 > ack ? 2 : 3;
+        S.h_head = slot(n);
+        S.h_n -= n;
+        if (n < 3)
+            return;
         while (S.h_n && hi[slot(0)] <= ack)
         {
             S.h_head = slot(1);
