@@ -1104,8 +1104,7 @@ TR_HD bool host_events(const RSim &s, int h, int64_t t, int64_t *wake, Due *due,
         h_collect_due(s, h, e.n, t1, due, &ndue);
     int ai = 0, di = 0;
     SArr a{};           // the next arrival
-    Chain ac;           // its chain (read when a tie or its event needs it)
-    bool have_a = false, have_ac = false;
+    bool have_a = false;
     int sf_at = -1, sf = -1;
     int64_t sf_t = INT64_MAX;
     unsigned long long n_ev = 0, n_arr = 0, n_ack = 0, n_data = 0;
@@ -1121,7 +1120,6 @@ TR_HD bool host_events(const RSim &s, int h, int64_t t, int64_t *wake, Due *due,
                 stage_arrival(s, a, (uint32_t)(abase + ai), lin, p);
             }
             have_a = true;
-            have_ac = false;
         }
         while (di < ndue && s.qp[due[di].flow].t[due[di].kind] != due[di].at)
             di++; // (stopped or moved)
@@ -1143,27 +1141,42 @@ TR_HD bool host_events(const RSim &s, int h, int64_t t, int64_t *wake, Due *due,
             tmin = ct[k] < tmin ? ct[k] : tmin;
         if (tmin == INT64_MAX)
             break;
-        if (ct[0] == tmin && !have_ac)
-        {
-            ld_chain(ac, &s.msg[a.frame].c);
-            have_ac = true;
-        }
-        auto chain_of = [&](int k) -> const Chain & {
-            return k == 0 ? ac : k == 1 ? s.h_tc[h] : k == 2 ? s.h_ns[h] : k == 3 ? s.qc[due[di].flow].c[due[di].kind] : s.flow[sf].start_chain;
-        };
-        int bk = -1;
+        int bk = -1, at = 0;
         for (int k = 0; k < 5; k++)
+            if (ct[k] == tmin)
+            {
+                bk = bk < 0 ? k : bk;
+                at++;
+            }
+        if (at > 1)
         {
-            if (ct[k] != tmin)
-                continue;
-            if (bk < 0 || runs_before(s, tmin, k == 0 ? a.acode : 0, chain_of(k), tmin, bk == 0 ? a.acode : 0, chain_of(bk)))
-                bk = k;
+            // a tie: the chains (copies that only a tie makes: what is chosen by reference lives in
+            // memory, and every event would wait for its own stores)
+            Chain ac;
+            if (ct[0] == tmin)
+                ld_chain(ac, &s.msg[a.frame].c);
+            auto chain_of = [&](int k) -> const Chain & {
+                return k == 0 ? ac : k == 1 ? s.h_tc[h] : k == 2 ? s.h_ns[h] : k == 3 ? s.qc[due[di].flow].c[due[di].kind] : s.flow[sf].start_chain;
+            };
+            for (int k = bk + 1; k < 5; k++)
+                if (ct[k] == tmin && runs_before(s, tmin, 0, chain_of(k), tmin, bk == 0 ? a.acode : 0, chain_of(bk)))
+                    bk = k;
         }
         e.now = tmin;
         if (bk == 0)
+        {
+            Chain ac;
+            ld_chain(ac, &s.msg[a.frame].c);
             chain_push(s, e.cur, a.acode, ac, e.n.tail);
+        }
+        else if (bk == 1)
+            e.cur = s.h_tc[h];
+        else if (bk == 2)
+            e.cur = s.h_ns[h];
+        else if (bk == 3)
+            e.cur = s.qc[due[di].flow].c[due[di].kind];
         else
-            e.cur = chain_of(bk);
+            e.cur = s.flow[sf].start_chain;
         e.ord = 0;
         n_ev++;
         if (bk == 0)
