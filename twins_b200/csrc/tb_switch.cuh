@@ -7,8 +7,7 @@
 // iteration of one loop moves one frame on every port at once, whether it starts on the wire or
 // joins the queue. (A serial loop per port of its own, each with its own start and enqueue loops,
 // ran the ports of a warp one after the other: with it a FatTree k=16 DCTCP world of 2,253 flows
-// took 207 ms, now 128 ms; 12 mixed leaf-spine worlds 633 ms, now 322 ms; 96 k=8 worlds 274 ms,
-// now 177 ms.) A slot whose messages exceed the staging area runs a port per lane in phases
+// took 207 ms, with this split 128 ms; 96 k=8 worlds 274 ms, with it 177 ms.) A slot whose messages exceed the staging area runs a port per lane in phases
 // through L2 (sw_phase_*).
 #pragma once
 #include "tb_slot.cuh"
