@@ -346,6 +346,8 @@ struct HostNic
                 break;
             Frame f;
             frame_copy(&f, start ? (size ? &ring[head] : &list[jq]) : &list[i]);
+            const bool kick = f.to_sender & OFFER_KICK;
+            f.to_sender &= 1; // (the list's mark is no part of the frame: not on the wire, not in the trace)
             if (!start)
                 offered++;
             const bool idle = waiting == 0 && busy <= ta && room;
@@ -365,7 +367,6 @@ struct HostNic
                 tx_len = f.len;
                 busy = began + tx_len * (int)PS_PER_BYTE;
                 f.ts = S0 + busy + PROP_PS;
-                f.to_sender &= 1;
                 frame_store_link(&msg[n_out++], f);
                 early += busy < SLOT;
                 if (!start)
@@ -388,7 +389,7 @@ struct HostNic
                 continue;
             }
             // an offer that finds the wire busy, or frames waiting
-            const bool woken = began < ta || ((f.to_sender & OFFER_KICK) && idle_at == ta);
+            const bool woken = began < ta || (kick && idle_at == ta);
             const int backlog = !waiting || busy <= ta ? waiting : waiting - (woken ? 1 : 0);
             bool gone = false;
             ovf += !room;
