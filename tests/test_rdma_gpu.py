@@ -67,3 +67,20 @@ def test_rdma_refusals(native_lib):
         with pytest.raises(api.TwinsError) as e:
             sim.add_rdma_world(cfg.replace("CC_MODE 3", "CC_MODE 2"), topo, flows)
         assert "CC_MODE" in str(e.value)
+
+
+def test_rdma_kept_batches_of_different_switches(native_lib):
+    """Two batches held at once whose switches differ in ports, so that their launches take different
+    amounts of shared memory: the one with more, prepared first, still runs after the other was prepared."""
+    names = ["ft8_incast32_hpcc", "ft4_incast15_hpcc"]
+    sims = []
+    for name in names:
+        sim = api.Simulator()
+        sim.add_rdma_world(*inputs(name))
+        sim.prepare()
+        sims.append(sim)
+    for name, sim in zip(names, sims):
+        assert sim.run() == api.TB_OK
+        _, fct = sim.rdma_results(0)
+        assert (fct == want(name, len(fct))).all(), name
+        sim.close()

@@ -164,6 +164,20 @@ static const void *rdma_kernel_of(int units, int sms)
     return units > 3 * sms && units <= 4 * sms ? (const void *)rdma_slot_kernel<4> : (const void *)rdma_slot_kernel<3>;
 }
 
+// A kernel's limit of dynamic shared memory belongs to the process, not to a batch: set to all that a
+// block may have, so that no batch's limit is lowered by the next one's.
+static cudaError_t allow_shared_memory(const void *kernel, int dev)
+{
+    cudaFuncAttributes a;
+    int most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+    return e;
+}
+
 int rdma_launch_shape(int max_deg, int units, int *grid, size_t *smem, const void **kernel)
 {
     *smem = block_scratch_bytes(max_deg);
@@ -171,7 +185,7 @@ int rdma_launch_shape(int max_deg, int units, int *grid, size_t *smem, const voi
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     *kernel = rdma_kernel_of(units, sms);
-    if (cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess)
+    if (allow_shared_memory(*kernel, dev) != cudaSuccess)
         return (int)cudaGetLastError();
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, *kernel, RDMA_WARPS * 32, *smem) != cudaSuccess)
         return (int)cudaGetLastError();
