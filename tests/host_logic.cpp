@@ -23,6 +23,8 @@ void hl_cand(int k, int *out)
 
 int hl_grid_of(long long units, int warps, int per_sm, int sms, int grid_req) { return grid_of(units, warps, per_sm, sms, grid_req); }
 
+int hl_rdma_four_blocks(long long units, int sms, int fit) { return rdma_four_blocks(units, sms, fit); }
+
 int hl_running_units(const int *alive, const int *worlds, int W, int lanes, int H, int *out, int cap)
 {
     std::vector<std::array<int, 4>> wr(W);

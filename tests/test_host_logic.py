@@ -28,6 +28,7 @@ def hl(tmp_path_factory):
         "hl_n_cand": (C.c_int, []),
         "hl_cand": (None, [C.c_int, C.POINTER(C.c_int)]),
         "hl_grid_of": (C.c_int, [ll, C.c_int, C.c_int, C.c_int, C.c_int]),
+        "hl_rdma_four_blocks": (C.c_int, [ll, C.c_int, C.c_int]),
         "hl_running_units": (C.c_int, [C.POINTER(C.c_int), C.POINTER(C.c_int), C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int), C.c_int]),
         "hl_tuner": (vp, [C.c_int, C.c_int, C.c_int, C.c_int, ll, C.c_int, ll, C.c_uint]),
         "hl_tuner_free": (None, [vp]),
@@ -79,6 +80,15 @@ def test_grid_rule(hl):
     assert g(10_000, 4, 2, 148, 0) == 296  # capped at what is co-resident
     assert g(10, 4, 0, 148, 0) == 0  # the shape does not fit
     assert g(10, 4, 2, 148, 50) == 50 and g(10, 4, 2, 148, 1000) == 296  # the caller's grid, capped
+
+
+def test_rdma_kernel_rule(hl):
+    """Four blocks per SM for RDMA batches of more units than three per SM hold and no more than four do, and
+    only where the batch's shared memory lets a fourth block be resident."""
+    four = hl.hl_rdma_four_blocks
+    assert [four(u, 148, 4) for u in (1, 444, 445, 592, 593, 896)] == [0, 0, 1, 1, 0, 0]
+    assert [four(u, 148, 3) for u in (1, 444, 445, 592, 593)] == [0, 0, 0, 0, 0]
+    assert [four(u, 132, 5) for u in (396, 397, 528, 529)] == [0, 1, 1, 0]
 
 
 def tuner(hl, entities, kmax=8, resident=1184, mask=0x1FF, autotune=True, fixed=(1, MID, 0)):

@@ -40,6 +40,18 @@ inline int grid_of(long long units, int warps, int per_sm, int sms, int grid_req
     return grid_req > 0 ? std::min(grid_req, most) : (int)std::min<long long>(need, most);
 }
 
+// Whether a batch of `units` RDMA units (a block each) runs the kernel of 128 registers, which spills and
+// of which `fit` blocks fit on an SM with the batch's shared memory, instead of the one of 168 registers,
+// three blocks per SM: where every unit then has a resident block of its own and with three it has not.
+// Measured on 148 SMs, three / four blocks per SM: k=8 worlds of 448 units 36.4 / 37.5 ms, 560 units 45.0 /
+// 40.9 ms, eight of them, 896 units, 279 / 293 ms; leaf-spines of 24 ports, 528 units, 35.6 / 33.7 ms; FatTree
+// k=16, 576 units, 33.8 / 30.7 ms. Switches of more than 26 ports leave room for three blocks only, and the
+// spills gain nothing: 30 ports, 564 units, 50.9 / 53.6 ms; 32 ports, 528 units, 59.3 / 62.3 ms.
+inline bool rdma_four_blocks(long long units, int sms, int fit)
+{
+    return fit >= 4 && units > 3LL * sms && units <= 4LL * sms;
+}
+
 // The units of a batch's running worlds, ascending: host units (`lanes` hosts each; a unit that
 // holds hosts of two worlds appears once, while either runs), then one unit per switch after
 // all host units. worlds[w] = {first host, hosts, first switch, switches}; alive(w) whether

@@ -5,6 +5,7 @@
 // bounded: a barrier that waits too long sets the run's error flag and the launch returns.
 // (reference: rdma_slot / rdma_persist / slot_end, src/rdma/rstep.cuh:3451-3577, 4020-4214)
 #include "tr_kernel.h"
+#include "tb_host.h"
 
 namespace tr
 {
@@ -156,14 +157,6 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32, MIN_BLOCKS) rdma_slot_kernel(
     }
 }
 
-// The kernel of `units` units: with 168 registers (3 blocks per SM), unless 128 (4 blocks, spilling) let
-// every unit have a resident block of its own and 168 do not. Measured, 3 / 4 blocks: FatTree k=16
-// (576 units) 91 / 85 ms; eight k=8 worlds (896 units) 279 / 293 ms.
-static const void *rdma_kernel_of(int units, int sms)
-{
-    return units > 3 * sms && units <= 4 * sms ? (const void *)rdma_slot_kernel<4> : (const void *)rdma_slot_kernel<3>;
-}
-
 // A kernel's limit of dynamic shared memory belongs to the process, not to a batch: set to all that a
 // block may have, so that no batch's limit is lowered by the next one's.
 static cudaError_t allow_shared_memory(const void *kernel, int dev)
@@ -184,11 +177,16 @@ int rdma_launch_shape(int max_deg, int units, int *grid, size_t *smem, const voi
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    *kernel = rdma_kernel_of(units, sms);
-    if (allow_shared_memory(*kernel, dev) != cudaSuccess)
-        return (int)cudaGetLastError();
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, *kernel, RDMA_WARPS * 32, *smem) != cudaSuccess)
-        return (int)cudaGetLastError();
+    // (the four-block kernel first: whether the batch's shared memory leaves room for its fourth block)
+    for (const void *k : {(const void *)rdma_slot_kernel<4>, (const void *)rdma_slot_kernel<3>})
+    {
+        *kernel = k;
+        if (allow_shared_memory(k, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, RDMA_WARPS * 32, *smem) != cudaSuccess)
+            return (int)cudaGetLastError();
+        if (tb::rdma_four_blocks(units, sms, per_sm))
+            break;
+    }
     if (per_sm < 1)
         return (int)cudaErrorInvalidConfiguration;
     // a block per unit (a group of NIC hosts or a switch) where they fit at once; else every
