@@ -46,3 +46,13 @@ def test_static_run_rejects_a_world_too_large(native_lib):
         api.run_world_static(w.topo, w.flows, w.params)
     assert e.value.code == -3
     assert "fixed area" in str(e.value)
+
+
+def test_static_run_holds_48600_connections(native_lib):
+    """The fixed area holds a FatTree k=4 world of 48,600 one-segment connections (its limit lies near 49,600:
+    what a connection's records take decides it)."""
+    i = np.arange(48_600)
+    flows = api.Flows.from_arrays(i % 16, (i % 16 + 1 + i // 16 % 15) % 16, np.full(len(i), 1000), 1000 + i * 100)
+    est, done, status = api.run_world_static(api.Topology.fattree(4), flows, api.TcpParams("newreno", 30, 200), max_slots=200)
+    assert status == api.TB_OK
+    assert (done >= 0).any() and (done[-1000:] == -1).all()

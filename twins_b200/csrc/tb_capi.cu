@@ -665,13 +665,13 @@ void build_image(const HostWorld &w, const Place &pl, WorldImage &img)
         RcvRec &R = img.rcv[cc];
         memset(&S_, 0, sizeof S_);
         memset(&R, 0, sizeof R);
-        S_.world = R.world = pl.world;
-        S_.src_local = R.src_local = first.src;
-        S_.dst_local = R.dst_local = first.dst;
+        // (host ids are 16-bit, as the frames that carry them)
+        S_.src_local = R.src_local = (uint16_t)first.src;
+        S_.dst_local = (uint16_t)first.dst;
         S_.hash_data = w.hash_data[cc];
-        S_.hash_ack = R.hash_ack = w.hash_ack[cc];
-        S_.up = S_.hash_data % (uint32_t)w.ecmp_n;
-        R.up_ack = R.hash_ack % (uint32_t)w.ecmp_n;
+        S_.hash_ack = w.hash_ack[cc];
+        S_.up = (uint16_t)(S_.hash_data % (uint32_t)w.ecmp_n);
+        R.up_ack = (uint16_t)(S_.hash_ack % (uint32_t)w.ecmp_n);
         S_.m_first = pl.msg0 + w.row_msg[cr[0]];
         S_.m_cnt = (int)cr.size();
         S_.fin_on = R.fin_on = (uint8_t)(w.p.fin != 0);

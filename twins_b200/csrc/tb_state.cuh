@@ -50,23 +50,23 @@ TB_HD uint32_t sent_list_cap(uint64_t segs)
 // The sending side of a connection (TcpSocketBase, TcpTxBuffer, the congestion control). A record has
 // a core, which every event of its connection works on in registers (tb_tcp.cuh: Snd, loaded when the
 // event begins and stored when it ends, in 16-byte words), and the rest, which few events touch and
-// which stays in memory. The core begins with what never changes, which is not stored back.
-constexpr int REC_FIXED = 48; // the bytes of both records' cores that never change
+// which stays in memory. The core begins with what never changes, which is not stored back (FIXED bytes).
+// Sizes are kept down, since a world's records count against the fixed area of tb_run_static, a context's
+// memory budget and a server's: 592 bytes a connection for both sides, with 9-run chains.
 struct alignas(16) SndCore
 {
+    static constexpr int FIXED = 32;
     // read-only
     uint64_t it_off;
-    int world, src_local, dst_local;
+    uint16_t src_local, dst_local;
+    uint16_t up;        // its data's ECMP choice: hash_data modulo the world's equal-cost uplinks
+    uint8_t fin_on, pad0;
     int m_first, m_cnt; // messages (global ids, consecutive)
     uint32_t it_cap;    // sent-list / RTT-history ring capacity
-    uint32_t up;        // its data's ECMP choice: hash_data modulo the world's equal-cost uplinks
-    // (while an event works on the core; 0 in memory) the flag word of the sent list stored last, its
-    // number + 1 and its value
-    uint32_t cw_at, cw;
-    uint32_t pad0;
+    uint32_t hash_data;
     // application and socket
     int m_due, m_wr, m_dn;
-    uint8_t st, cong, fin, fin_on;
+    uint8_t st, cong, fin, cub_found;
     uint32_t tail, una, nxt, high;
     uint32_t cwnd, ssthresh, dupacks;
     uint32_t it_head, it_n, h_head, h_n;
@@ -83,10 +83,9 @@ struct alignas(16) SndCore
 };
 struct SndRec : SndCore
 {
-    uint32_t hash_data, hash_ack;
-    // TcpCubic
+    uint32_t hash_ack;
+    // TcpCubic (and cub_found)
     uint32_t cub_cnt, cub_lastmax, cub_origin, cub_endseq, cub_samples, cub_ackcnt, cub_tcpcwnd;
-    uint8_t cub_found, pad1[3];
     double cub_k;
     int64_t cub_delaymin, cub_epoch, cub_roundstart, cub_lastack, cub_currrtt;
     Chain rchain; // the retransmission (or SYN) timer's
@@ -96,24 +95,23 @@ struct SndRec : SndCore
 // the receiving side (TcpRxBuffer, delayed ACKs, DCTCP's CE state, the closing states)
 struct alignas(16) RcvCore
 {
+    static constexpr int FIXED = 16;
     uint64_t oo_off;
-    int world, src_local, dst_local;
-    uint32_t hash_ack;
     uint32_t oo_cap;
     uint32_t bytes;             // the connection's bytes (all its messages)
-    uint32_t up_ack;            // its ACKs' ECMP choice
-    uint32_t pad0[3];
+    uint16_t src_local;
+    uint16_t up_ack;            // its ACKs' ECMP choice
     uint8_t fin_on, up, est, st;
     uint32_t rcv_nxt, ooo_n, ooo_h, prior_rcv_nxt;
-    uint8_t last_n, syn_n, delack_count, ce_state, prior_flag, reserved, ecn_r, pad1;
-    uint32_t pad2;
-    int64_t fin_seq, synack_t, srtt, rttvar, last_at, frx_at, syn_at, delack_at, ecn_ce_seq, pad3;
+    uint8_t last_n, syn_n, delack_count, ce_state, prior_flag, reserved, ecn_r, pad0;
+    int64_t fin_seq, synack_t, srtt, rttvar, last_at, frx_at, syn_at, delack_at, ecn_ce_seq, pad1;
 };
 struct RcvRec : RcvCore
 {
     Chain dchain; // delayed ACK, SYN-ACK retransmission, LastAckTimeout
     Chain fchain; // the FIN+ACK's own retransmission
 };
+static_assert(sizeof(SndRec) + sizeof(RcvRec) == 432 + 4 * sizeof(Chain), "a connection's records");
 
 struct MsgRec
 {

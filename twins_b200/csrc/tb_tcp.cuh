@@ -51,13 +51,19 @@ struct HostCtx
 // sender's and the receiver's record last used stay in registers from event to event (Recs): most of
 // a busy host's events in a slot are one connection's, and loading a record that the event before
 // has just stored waits 600 cycles for the stores.
+struct FlagWord // a flag word of a sent list: its number + 1 (0: none) and its value
+{
+    uint32_t at, w;
+};
 struct Snd : SndCore
 {
+    FlagWord kept; // the flag word stored last (SentList)
     SndRec *rec;
     int f; // the connection (-1: none)
     TB_D Snd() : f(-1) {}
     TB_D void load(SndRec &r, int flow)
     {
+        kept = {0, 0};
         rec = &r;
         f = flow;
         load_core<SndCore>(this, &r);
@@ -82,7 +88,7 @@ struct Snd : SndCore
         const uint4 *a = reinterpret_cast<const uint4 *>(from);
         uint4 *b = reinterpret_cast<uint4 *>(to);
 #pragma unroll
-        for (int i = REC_FIXED / 16; i < (int)(sizeof(Core) / 16); i++)
+        for (int i = Core::FIXED / 16; i < (int)(sizeof(Core) / 16); i++)
             b[i] = a[i];
     }
 };
@@ -99,7 +105,8 @@ struct Rcv : RcvCore
     }
     TB_D void store() const { Snd::store_core<RcvCore>(rec, this); }
 };
-static_assert(offsetof(SndCore, m_due) == REC_FIXED && offsetof(RcvCore, fin_on) == REC_FIXED && sizeof(SndCore) % 16 == 0 && sizeof(RcvCore) % 16 == 0,
+static_assert(offsetof(SndCore, m_due) == SndCore::FIXED && offsetof(RcvCore, src_local) == RcvCore::FIXED && sizeof(SndCore) % 16 == 0 &&
+                  sizeof(RcvCore) % 16 == 0,
               "cores move as 16-byte words");
 
 template <bool KEEP>
@@ -260,18 +267,21 @@ struct SentList
     uint32_t *start;
     uint32_t *fw; // flag words
     uint32_t cap;
+    FlagWord own, &kept; // the word stored last: kept with the record while events work on it, else the list's own
 
-    // A flag word, and its store. The word stored last is kept with the record's core: an append reads
-    // the word that the append before it stored, and a load of a line just stored waits for the store.
-    TB_D uint32_t word(uint32_t w) const { return w + 1 == S.cw_at ? S.cw : fw[w]; }
+    // A flag word, and its store. An append reads the word that the append before it stored, and a load
+    // of a line just stored waits for the store.
+    TB_D uint32_t word(uint32_t w) const { return w + 1 == kept.at ? kept.w : fw[w]; }
     TB_D void set_word(uint32_t w, uint32_t v)
     {
         fw[w] = v;
-        S.cw_at = w + 1;
-        S.cw = v;
+        kept = {w + 1, v};
     }
 
-    TB_D SentList(const Sim &s, SndCore &S_) : S(S_)
+    TB_D SentList(const Sim &s, Snd &S_) : SentList(s, S_, S_.kept) {}
+    TB_D SentList(const Sim &s, SndRec &S_) : SentList(s, S_, own) { own = {0, 0}; }
+    SentList(const SentList &) = delete;
+    TB_D SentList(const Sim &s, SndCore &S_, FlagWord &kept_) : S(S_), kept(kept_)
     {
         start = s.it_start + S.it_off;
         fw = reinterpret_cast<uint32_t *>(s.it_fl + S.it_off);
@@ -870,20 +880,20 @@ TB_D void on_acked(Snd &S, int64_t now)
     if (S.rec->cub_delaymin == INT64_MIN || S.rec->cub_delaymin > rtt)
         S.rec->cub_delaymin = rtt;
     const uint32_t w = S.cwnd;
-    if (S.rec->cub_found || w > S.ssthresh || w < 16 * MSS)
+    if (S.cub_found || w > S.ssthresh || w < 16 * MSS)
         return;
     if (now - S.rec->cub_lastack <= ACK_DELTA)
     {
         S.rec->cub_lastack = now;
         if (now - S.rec->cub_roundstart > S.rec->cub_delaymin)
-            S.rec->cub_found = 1;
+            S.cub_found = 1;
     }
     if (S.rec->cub_samples >= 8)
     {
         const int64_t dm = S.rec->cub_delaymin;
         const int64_t slack = dm < DELAY_MIN ? DELAY_MIN : dm > DELAY_MAX ? DELAY_MAX : dm;
         if (S.rec->cub_currrtt > dm + slack)
-            S.rec->cub_found = 1;
+            S.cub_found = 1;
     }
     else
     {
@@ -891,7 +901,7 @@ TB_D void on_acked(Snd &S, int64_t now)
             S.rec->cub_currrtt = rtt;
         S.rec->cub_samples++;
     }
-    if (S.rec->cub_found)
+    if (S.cub_found)
         S.ssthresh = w;
 }
 // IncreaseWindow: slow start by whole segments, else one segment per acks_per_segment ACKs
@@ -934,7 +944,7 @@ TB_D void on_loss(Snd &S, int64_t now)
     S.rec->cub_ackcnt = 0;
     S.rec->cub_tcpcwnd = 0;
     S.rec->cub_delaymin = INT64_MIN;
-    S.rec->cub_found = 0;
+    S.cub_found = 0;
     new_round(S, now);
 }
 } // namespace cubic
