@@ -186,9 +186,9 @@ int tb_get_stats(tb_ctx *ctx, tb_stats *out);
 /* Launch shape: hosts per warp (1..32) and the grid (0: chosen from occupancy); turns autotuning
  * off. Replaces the reference's --host_lanes (src/main.cu:183-184, 523-526). */
 int tb_set_launch(tb_ctx *ctx, int host_lanes, int grid);
-/* The same with the frames a warp stages in shared memory per slot (1..384, 1..256 in the 25-run
- * build; default 192; fewer leave room for more resident blocks per SM, more stage the slots of
- * big switches). */
+/* The same with the frames arriving in a slot that a warp stages in shared memory (1..384, 1..256 in
+ * the 25-run build; default 192). A slot of more frames is run from L2. Fewer leave more of the SM's
+ * memory to L1 and to resident blocks, more stage the slots of big switches. */
 int tb_set_launch_shape(tb_ctx *ctx, int host_lanes, int stage_frames, int grid);
 /* A label of a fixed shape (one host per warp only), reported back in tb_stats. Every shape keeps
  * a switch port's slot state on chip; the label changes neither results nor speed. */

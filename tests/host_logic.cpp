@@ -9,7 +9,7 @@ extern "C" {
 
 int hl_stage(int which)
 {
-    const int v[4] = {SW_STAGE_SMALL, SW_STAGE, SW_STAGE_TWO, SW_STAGE_MAX};
+    const int v[6] = {STAGE_SMALL, STAGE_MID, STAGE_TWO, STAGE_BIG, SW_STAGE, SW_STAGE_MAX};
     return v[which];
 }
 

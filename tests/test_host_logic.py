@@ -57,11 +57,12 @@ def hl(tmp_path_factory):
     return lib
 
 
-SMALL, MID, TWO, MAX = 96, 192, 288, 384
+SMALL, MID, TWO, BIG = 72, 144, 216, 288  # the tuner's staging areas, frames
 
 
 def test_staging_sizes_and_candidates(hl):
-    assert [hl.hl_stage(i) for i in range(4)] == [SMALL, MID, TWO, MAX]
+    assert [hl.hl_stage(i) for i in range(4)] == [SMALL, MID, TWO, BIG]
+    assert [hl.hl_stage(i) for i in (4, 5)] == [192, 384]  # a fixed shape's default, and the most it may ask for
     cands = []
     for k in range(hl.hl_n_cand()):
         v = (C.c_int * 3)()
@@ -69,7 +70,7 @@ def test_staging_sizes_and_candidates(hl):
         cands.append(tuple(v))
     assert len(set(cands)) == len(cands)
     for lanes, stage, pl in cands:
-        assert lanes in (1, 4, 32) and 1 <= stage <= MAX
+        assert lanes in (1, 4, 32) and 1 <= stage <= BIG
         assert not pl or lanes == 1  # the port-local egress runs with one host per warp only
 
 
@@ -108,7 +109,7 @@ def test_tuner_start_rule(hl):
     hl.hl_tuner_free(t)
     # big switches: the port-local egress with the largest staging
     t, shapes = tuner(hl, 208, kmax=16)
-    assert shapes[hl.hl_tuner_best(t)][:3] == (1, MAX, 1)
+    assert shapes[hl.hl_tuner_best(t)][:3] == (1, BIG, 1)
     hl.hl_tuner_free(t)
     # many entities: 32 hosts per warp with the smallest staging (the rule is on entities <= 2x resident)
     t, shapes = tuner(hl, 2 * 1184 + 1, kmax=32)

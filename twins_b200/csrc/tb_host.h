@@ -16,18 +16,17 @@
 namespace tb
 {
 
-// frames a warp stages in shared memory per switch (or host) and slot: the default staging area
-// and the largest; a launch may use a smaller one (more resident warps per SM, fewer slots
-// staged) or a larger one (big switches' slots staged, fewer resident warps)
+// The staging area: the frames arriving in a slot that a warp copies to shared memory, per switch (or
+// host); a slot of more frames is run from L2. A fixed launch shape's default and the most that one may
+// ask for (a block's four warps then take 123 KB, in the 25-run build, whose frames are larger, 154 KB).
 constexpr int SW_STAGE = 192;
-constexpr int SW_STAGE_MAX = TB_CHAIN_RUNS > 9 ? 256 : 384; // (what four warps' scratch fits in 227 KB)
-constexpr int SW_STAGE_SMALL = 96;
-constexpr int SW_STAGE_TWO = 288; // two blocks of four warps fit on an SM with it
-
-// The staging area of a launch shape's `stage` frames. A shape counts the frames of two slots' link
-// messages, of which a reader takes about half (the late frames of the one, the early ones of the
-// other); the area holds three quarters of them.
-inline int stage_area(int stage) { return stage * 3 / 4 > 1 ? stage * 3 / 4 : 1; }
+constexpr int SW_STAGE_MAX = TB_CHAIN_RUNS > 9 ? 256 : 384;
+// The areas the tuner chooses among. What a block's area leaves of the SM's 256 KB is L1, which holds
+// the units' records, so the first choice is not the largest: with one host per warp two blocks of 216
+// frames (145 KB) leave more than 100 KB.
+constexpr int STAGE_SMALL = 72, STAGE_MID = 144;
+constexpr int STAGE_TWO = TB_CHAIN_RUNS > 9 ? STAGE_MID : 216;
+constexpr int STAGE_BIG = TB_CHAIN_RUNS > 9 ? 192 : 288;
 
 // the grid of a launch: a block per `warps` units, at most what is co-resident (per_sm blocks on
 // each of sms SMs; 0: the shape does not fit), or the caller's grid when it asked for one
@@ -125,9 +124,8 @@ struct ShapeTuner
 
     // the candidates: (lanes, stage, port-local)
     static constexpr int N_CAND = 9;
-    static constexpr int CAND[N_CAND][3] = {{1, SW_STAGE_TWO, 0},  {1, SW_STAGE, 0},       {4, SW_STAGE, 0},
-                                            {32, SW_STAGE, 0},     {1, SW_STAGE_SMALL, 0}, {32, SW_STAGE_SMALL, 0},
-                                            {1, SW_STAGE_MAX, 0},  {1, SW_STAGE_MAX, 1},   {1, SW_STAGE_TWO - 32, 1}};
+    static constexpr int CAND[N_CAND][3] = {{1, STAGE_TWO, 0},   {1, STAGE_MID, 0},   {4, STAGE_MID, 0}, {32, STAGE_MID, 0}, {1, STAGE_SMALL, 0},
+                                            {32, STAGE_SMALL, 0}, {1, STAGE_BIG, 0}, {1, STAGE_BIG, 1}, {1, 192, 1}};
 
     // autotune: probe the candidates that fit (fits(lanes, stage, port_local) on this device),
     // else run the one shape (lanes, stage, port_local). entities: hosts and switches to run;
@@ -151,7 +149,7 @@ struct ShapeTuner
             // staging, for four blocks per SM)
             const int lanes0 = entities <= 2 * resident ? 1 : 32;
             const bool pl0 = lanes0 == 1 && kmax >= 16;
-            const int stage0 = lanes0 == 1 ? (pl0 ? SW_STAGE_MAX : SW_STAGE_TWO) : SW_STAGE_SMALL;
+            const int stage0 = lanes0 == 1 ? (pl0 ? STAGE_BIG : STAGE_TWO) : STAGE_SMALL;
             for (size_t k = 0; k < shapes.size(); k++)
                 if (shapes[k].lanes == lanes0 && shapes[k].stage == stage0 && shapes[k].port_local == pl0)
                     best = k;

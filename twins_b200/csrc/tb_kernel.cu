@@ -604,6 +604,10 @@ __device__ __forceinline__ bool switch_step(const Sim &s, int sw, int64_t gt, in
     else
     {
         __syncwarp();
+#ifdef TB_QTRACE
+        if (lane == 0)
+            ev_add(s, sr.world, EV_UNSTAGED, 1);
+#endif
         // (copies: what a call is given the address of lives in memory, and the staged slot's is to stay
         // in registers)
         const SwCtx y = x;
@@ -895,7 +899,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
 }
 
 // dynamic shared memory of a block: one switch scratch (with its staging area) per warp
-static size_t smem_bytes(int stage_cap) { return sw_shared_bytes(stage_area(stage_cap)) * WARPS_PER_BLOCK; }
+static size_t smem_bytes(int stage_cap) { return sw_shared_bytes(stage_cap) * WARPS_PER_BLOCK; }
 
 // the instantiation of a launch shape: several hosts per warp or one host per warp; each with the
 // grid barrier or without (F_*: batches)
@@ -983,8 +987,7 @@ int launch_slots(const Sim &s, int grid, int max_slots_per_launch, int host_lane
     const int k = kind_of(host_lanes);
     if (!smem_attr(k) || stage_cap < 1 || stage_cap > SW_STAGE_MAX)
         return (int)cudaErrorInvalidValue;
-    int area = stage_area(stage_cap);
-    void *args[] = {(void *)&s, (void *)&max_slots_per_launch, (void *)&host_lanes, (void *)&area};
+    void *args[] = {(void *)&s, (void *)&max_slots_per_launch, (void *)&host_lanes, (void *)&stage_cap};
     return launch_kind(k, args, grid, stage_cap, stream);
 }
 
@@ -998,8 +1001,7 @@ int launch_free(const Sim &s, int grid, int slots_per_world, int host_lanes, int
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return (int)e;
-    int area = stage_area(stage_cap);
-    void *args[] = {(void *)&s, (void *)&host_lanes, (void *)&area};
+    void *args[] = {(void *)&s, (void *)&host_lanes, (void *)&stage_cap};
     return launch_kind(k, args, grid, stage_cap, stream);
 }
 

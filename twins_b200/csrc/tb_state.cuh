@@ -168,6 +168,7 @@ enum : int
     EV_BARRIER_TIMEOUT,
     EV_HOST_SND,    // packet-events at hosts that reach a connection's sending side
     EV_HOST_FRAMES, // frames hosts emitted
+    EV_UNSTAGED,    // (trace build) switch slots of more frames than the staging area holds
     EV_N = 16
 };
 
