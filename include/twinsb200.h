@@ -85,7 +85,7 @@ typedef struct tb_stats
     int grid, host_lanes, warps_per_block; /* the launch shape that ran the most slots */
     int stage_frames;        /* frames a warp stages in shared memory in that shape */
     int autotuned;           /* 1: the shape was picked per launch by measured throughput */
-    int port_local;          /* that shape's label (tb_set_port_local) */
+    int port_local;          /* a fixed shape's label (tb_set_port_local); 0 when autotuned */
     long long graph_launches; /* launches replayed from a captured CUDA graph */
 } tb_stats;
 

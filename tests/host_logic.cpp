@@ -17,7 +17,7 @@ int hl_n_cand() { return ShapeTuner::N_CAND; }
 
 void hl_cand(int k, int *out)
 {
-    for (int i = 0; i < 3; i++)
+    for (int i = 0; i < 2; i++)
         out[i] = ShapeTuner::CAND[k][i];
 }
 
@@ -37,12 +37,12 @@ int hl_running_units(const int *alive, const int *worlds, int W, int lanes, int 
     return (int)v.size();
 }
 
-void *hl_tuner(int autotune, int lanes, int stage, int port_local, long long entities, int kmax, long long resident, unsigned fits_mask)
+void *hl_tuner(int autotune, int lanes, int stage, long long entities, int kmax, long long resident, unsigned fits_mask)
 {
     auto *t = new ShapeTuner;
-    t->init(autotune != 0, lanes, stage, port_local != 0, entities, kmax, resident, [fits_mask](int l, int st, bool pl) {
+    t->init(autotune != 0, lanes, stage, entities, kmax, resident, [fits_mask](int l, int st) {
         for (int k = 0; k < ShapeTuner::N_CAND; k++)
-            if (ShapeTuner::CAND[k][0] == l && ShapeTuner::CAND[k][1] == st && (ShapeTuner::CAND[k][2] != 0) == pl)
+            if (ShapeTuner::CAND[k][0] == l && ShapeTuner::CAND[k][1] == st)
                 return ((fits_mask >> k) & 1) != 0;
         return false;
     });
@@ -52,14 +52,13 @@ void *hl_tuner(int autotune, int lanes, int stage, int port_local, long long ent
 void hl_tuner_free(void *t) { delete (ShapeTuner *)t; }
 int hl_tuner_n(void *t) { return (int)((ShapeTuner *)t)->shapes.size(); }
 
-// (lanes, stage, port_local, strikes)
+// (lanes, stage, strikes)
 void hl_tuner_shape(void *t, int k, int *out)
 {
     const ShapeTuner::Shape &s = ((ShapeTuner *)t)->shapes[k];
     out[0] = s.lanes;
     out[1] = s.stage;
-    out[2] = s.port_local;
-    out[3] = s.strikes;
+    out[2] = s.strikes;
 }
 
 int hl_tuner_best(void *t) { return (int)((ShapeTuner *)t)->best; }

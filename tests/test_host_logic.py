@@ -30,7 +30,7 @@ def hl(tmp_path_factory):
         "hl_grid_of": (C.c_int, [ll, C.c_int, C.c_int, C.c_int, C.c_int]),
         "hl_rdma_four_blocks": (C.c_int, [ll, C.c_int, C.c_int]),
         "hl_running_units": (C.c_int, [C.POINTER(C.c_int), C.POINTER(C.c_int), C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int), C.c_int]),
-        "hl_tuner": (vp, [C.c_int, C.c_int, C.c_int, C.c_int, ll, C.c_int, ll, C.c_uint]),
+        "hl_tuner": (vp, [C.c_int, C.c_int, C.c_int, ll, C.c_int, ll, C.c_uint]),
         "hl_tuner_free": (None, [vp]),
         "hl_tuner_n": (C.c_int, [vp]),
         "hl_tuner_shape": (None, [vp, C.c_int, C.POINTER(C.c_int)]),
@@ -65,13 +65,12 @@ def test_staging_sizes_and_candidates(hl):
     assert [hl.hl_stage(i) for i in (4, 5)] == [192, 384]  # a fixed shape's default, and the most it may ask for
     cands = []
     for k in range(hl.hl_n_cand()):
-        v = (C.c_int * 3)()
+        v = (C.c_int * 2)()
         hl.hl_cand(k, v)
         cands.append(tuple(v))
-    assert len(set(cands)) == len(cands)
-    for lanes, stage, pl in cands:
+    assert len(set(cands)) == len(cands)  # (no two launch the same kernel with the same staging)
+    for lanes, stage in cands:
         assert lanes in (1, 4, 32) and 1 <= stage <= BIG
-        assert not pl or lanes == 1  # the port-local egress runs with one host per warp only
 
 
 def test_grid_rule(hl):
@@ -92,43 +91,42 @@ def test_rdma_kernel_rule(hl):
     assert [four(u, 132, 5) for u in (396, 397, 528, 529)] == [0, 1, 1, 0]
 
 
-def tuner(hl, entities, kmax=8, resident=1184, mask=0x1FF, autotune=True, fixed=(1, MID, 0)):
-    t = hl.hl_tuner(int(autotune), fixed[0], fixed[1], fixed[2], entities, kmax, resident, mask)
+def tuner(hl, entities, kmax=8, resident=1184, mask=0xFF, autotune=True, fixed=(1, MID)):
+    t = hl.hl_tuner(int(autotune), fixed[0], fixed[1], entities, kmax, resident, mask)
     shapes = []
     for k in range(hl.hl_tuner_n(t)):
-        v = (C.c_int * 4)()
+        v = (C.c_int * 3)()
         hl.hl_tuner_shape(t, k, v)
         shapes.append(tuple(v))
     return t, shapes
 
 
 def test_tuner_start_rule(hl):
-    # few entities for the resident warps: one host per warp, two blocks per SM
-    t, shapes = tuner(hl, 208)
-    assert len(shapes) == 9 and shapes[hl.hl_tuner_best(t)][:3] == (1, TWO, 0)
-    hl.hl_tuner_free(t)
-    # big switches: the port-local egress with the largest staging
-    t, shapes = tuner(hl, 208, kmax=16)
-    assert shapes[hl.hl_tuner_best(t)][:3] == (1, BIG, 1)
-    hl.hl_tuner_free(t)
-    # many entities: 32 hosts per warp with the smallest staging (the rule is on entities <= 2x resident)
-    t, shapes = tuner(hl, 2 * 1184 + 1, kmax=32)
-    assert shapes[hl.hl_tuner_best(t)][:3] == (32, SMALL, 0)
-    hl.hl_tuner_free(t)
-    t, shapes = tuner(hl, 2 * 1184)
-    assert shapes[hl.hl_tuner_best(t)][:3] == (1, TWO, 0)
-    hl.hl_tuner_free(t)
+    def start(entities, **kw):
+        t, shapes = tuner(hl, entities, **kw)
+        assert len(shapes) == 8
+        best = shapes[hl.hl_tuner_best(t)][:2]
+        hl.hl_tuner_free(t)
+        return best
+
+    # few entities for the resident warps: one host per warp, two blocks per SM; big switches: the largest staging
+    assert start(208) == (1, TWO)
+    assert start(208, kmax=16) == (1, BIG)
+    # up to twice the resident warps; beyond, 32 hosts per warp with the smallest staging
+    assert start(2 * 1184) == (1, TWO)
+    assert start(2 * 1184 + 1) == (32, SMALL)
+    assert start(2 * 1184 + 1, kmax=32) == (32, SMALL)
 
 
 def test_tuner_candidates_that_fit_and_fixed_shape(hl):
     # only the candidates the device fits are kept; a start shape that does not fit falls back to the first
     t, shapes = tuner(hl, 208, mask=0b0000_1110)
-    assert [s[:3] for s in shapes] == [(1, MID, 0), (4, MID, 0), (32, MID, 0)] and hl.hl_tuner_best(t) == 0
+    assert [s[:2] for s in shapes] == [(1, MID), (4, MID), (32, MID)] and hl.hl_tuner_best(t) == 0
     hl.hl_tuner_free(t)
     # no autotuning, or nothing fits: the caller's shape alone, never probed
     for kw in ({"autotune": False}, {"mask": 0}):
-        t, shapes = tuner(hl, 208, fixed=(4, SMALL, 0), **kw)
-        assert [s[:3] for s in shapes] == [(4, SMALL, 0)]
+        t, shapes = tuner(hl, 208, fixed=(4, SMALL), **kw)
+        assert [s[:2] for s in shapes] == [(4, SMALL)]
         for _ in range(100):
             hl.hl_tuner_tick(t)
         assert not hl.hl_tuner_explore(t)

@@ -468,7 +468,7 @@ struct tb_ctx
     unsigned long long qtrace_cap = 0; // the enqueue trace (trace build): records kept, window (ps)
     long long qtrace_from = 0, qtrace_until = 0;
     bool autotune = true;         // pick the launch shape per launch by measured throughput
-    bool port_local = false;      // a fixed shape's switch egress (tb_set_port_local)
+    bool port_local = false;      // a fixed shape's label (tb_set_port_local)
     int dev_sms = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, la = nullptr, lb = nullptr;
@@ -806,8 +806,7 @@ void tuner_init(ShapeTuner &tu, const tb_ctx *c, bool autotune, int lanes, int s
     // 4,992 and 6,656 entities, 51 / 69, 67 / 77 and 82 / 78 ms: the line lies near 5,300 entities, four and a
     // half times the warps co-resident at one host per warp)
     const long long resident = (long long)c->dev_sms * std::max(1, tb::slot_kernel_blocks_per_sm(SW_STAGE, 1)) * TB_WARPS_PER_BLOCK * 9 / 4;
-    tu.init(autotune, lanes, stage, c->port_local, entities, kmax, resident,
-            [c](int l, int st, bool) { return grid_for(c, l, st) > 0; });
+    tu.init(autotune, lanes, stage, entities, kmax, resident, [c](int l, int st) { return grid_for(c, l, st) > 0; });
 }
 
 int prepare(tb_ctx *c)
@@ -1376,7 +1375,7 @@ int tb_run(tb_ctx *ctx, long long max_slots)
     st.warps_per_block = TB_WARPS_PER_BLOCK;
     st.stage_frames = most.stage;
     st.autotuned = tu.shapes.size() > 1;
-    st.port_local = most.port_local && most.lanes == 1;
+    st.port_local = !ctx->autotune && ctx->port_local && most.lanes == 1;
     st.graph_launches = graph.replays;
     st.bytes_d2h = 0;
     if (ctl.error)

@@ -96,11 +96,11 @@ void world_units(Alive alive, const std::vector<std::array<int, 4>> &worlds, int
     }
 }
 
-// Launch-shape autotuning, for tb_run and the server. A shape is the hosts per warp, the frames a
-// warp stages per slot and the switch egress variant; no shape changes a result. It starts from
-// one host per warp while the entities fit the resident warps about twice (latency-bound: each
-// host's serial events are the slot's critical path), else 32 hosts per warp (throughput-bound:
-// the lanes' memory accesses overlap). Every `period` launches each shape still in the running
+// Launch-shape autotuning, for tb_run and the server. A shape is the hosts per warp and the frames a
+// warp stages per slot; no shape changes a result. It starts from one host per warp while the
+// entities fit the resident warps about twice (latency-bound: each host's serial
+// events are the slot's critical path), else 32 hosts per warp (throughput-bound: the lanes' memory
+// accesses overlap). Every `period` launches each shape still in the running
 // runs a probe of `probe` slots, and one whose device time per slot beats the current one's by
 // more than 5% takes over; a shape that loses a probe by more than 30% twice, or by more than 60%
 // once, is not probed again until every fourth round of probes, which probes all shapes (the load changes along a run).
@@ -114,7 +114,6 @@ struct ShapeTuner
         int lanes, stage;
         long long slots;
         int strikes;
-        bool port_local; // (every shape keeps a port's slot state on chip: a label of the shape)
     };
     std::vector<Shape> shapes;
     size_t best = 0;
@@ -122,17 +121,16 @@ struct ShapeTuner
     int period = 12, probe = 128;
     int period0 = 12, most_period = 0; // (backoff: the first period and the bound; 0: none)
 
-    // the candidates: (lanes, stage, port-local)
-    static constexpr int N_CAND = 9;
-    static constexpr int CAND[N_CAND][3] = {{1, STAGE_TWO, 0},   {1, STAGE_MID, 0},   {4, STAGE_MID, 0}, {32, STAGE_MID, 0}, {1, STAGE_SMALL, 0},
-                                            {32, STAGE_SMALL, 0}, {1, STAGE_BIG, 0}, {1, STAGE_BIG, 1}, {1, 192, 1}};
+    // the candidates: (lanes, stage). (The 25-run build's sizes coincide for some: each shape is taken once.)
+    static constexpr int N_CAND = 8;
+    static constexpr int CAND[N_CAND][2] = {{1, STAGE_TWO},   {1, STAGE_MID},    {4, STAGE_MID}, {32, STAGE_MID},
+                                            {1, STAGE_SMALL}, {32, STAGE_SMALL}, {1, STAGE_BIG}, {1, 192}};
 
-    // autotune: probe the candidates that fit (fits(lanes, stage, port_local) on this device),
-    // else run the one shape (lanes, stage, port_local). entities: hosts and switches to run;
-    // resident: the warps co-resident on the device at one host per warp and the default
-    // staging; kmax: the most ports a switch has.
+    // autotune: probe the candidates that fit (fits(lanes, stage) on this device), else run the one
+    // shape (lanes, stage). entities: hosts and switches to run; resident: the warps co-resident on
+    // the device at one host per warp and the default staging; kmax: the most ports a switch has.
     template <class Fits>
-    void init(bool autotune, int lanes, int stage, bool port_local, long long entities, int kmax, long long resident, Fits fits)
+    void init(bool autotune, int lanes, int stage, long long entities, int kmax, long long resident, Fits fits)
     {
         shapes.clear();
         best = 0;
@@ -141,21 +139,19 @@ struct ShapeTuner
         if (autotune)
         {
             for (auto &x : CAND)
-                if (fits(x[0], x[1], x[2] != 0))
-                    shapes.push_back({x[0], x[1], 0, 0, x[2] != 0});
-            // (one host per warp: with big switches (16 ports or more), whose ports'
-            // enqueues are the critical path, the largest staging (and its label); else
-            // the largest staging that keeps two blocks per SM. 32 hosts per warp: the smallest
-            // staging, for four blocks per SM)
+                if (fits(x[0], x[1]) &&
+                    std::none_of(shapes.begin(), shapes.end(), [&](const Shape &y) { return y.lanes == x[0] && y.stage == x[1]; }))
+                    shapes.push_back({x[0], x[1], 0, 0});
+            // (one host per warp: with big switches (16 ports or more) the largest staging, else the one
+            // that leaves more to L1. 32 hosts per warp: the smallest)
             const int lanes0 = entities <= 2 * resident ? 1 : 32;
-            const bool pl0 = lanes0 == 1 && kmax >= 16;
-            const int stage0 = lanes0 == 1 ? (pl0 ? STAGE_BIG : STAGE_TWO) : STAGE_SMALL;
+            const int stage0 = lanes0 == 1 ? (kmax >= 16 ? STAGE_BIG : STAGE_TWO) : STAGE_SMALL;
             for (size_t k = 0; k < shapes.size(); k++)
-                if (shapes[k].lanes == lanes0 && shapes[k].stage == stage0 && shapes[k].port_local == pl0)
+                if (shapes[k].lanes == lanes0 && shapes[k].stage == stage0)
                     best = k;
         }
         if (shapes.empty())
-            shapes.push_back({lanes, stage, 0, 0, port_local});
+            shapes.push_back({lanes, stage, 0, 0});
     }
     // the period doubles after each round that keeps the shape, up to `most` launches
     void backoff(int most)
