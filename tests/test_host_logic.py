@@ -112,10 +112,11 @@ def test_tuner_start_rule(hl):
     # few entities for the resident warps: one host per warp, two blocks per SM; big switches: the largest staging
     assert start(208) == (1, TWO)
     assert start(208, kmax=16) == (1, BIG)
-    # up to twice the resident warps; beyond, 32 hosts per warp with the smallest staging
-    assert start(2 * 1184) == (1, TWO)
-    assert start(2 * 1184 + 1) == (32, SMALL)
-    assert start(2 * 1184 + 1, kmax=32) == (32, SMALL)
+    # up to four and a half times the resident warps; beyond, 32 hosts per warp with the smallest staging
+    assert start(1184 * 9 // 2) == (1, TWO)
+    assert start(1184 * 9 // 2 + 1) == (32, SMALL)
+    assert start(1184 * 9 // 2 + 1, kmax=32) == (32, SMALL)
+    assert start(4, resident=1) == (1, TWO) and start(5, resident=1) == (32, SMALL)
 
 
 def test_tuner_candidates_that_fit_and_fixed_shape(hl):

@@ -801,11 +801,7 @@ int grid_for(const tb_ctx *c, int host_lanes, int stage, int units = -1, bool fr
 // co-resident at one host per warp and the default staging
 void tuner_init(ShapeTuner &tu, const tb_ctx *c, bool autotune, int lanes, int stage, long long entities, int kmax = 0)
 {
-    // (the tuner starts with one host per warp up to twice the warps given here. Measured, one / 32 hosts
-    // per warp: 12 leaf-spine worlds, 2,940 entities, 178 / 417 ms; 16, 24 and 32 worlds of k=8, 3,328,
-    // 4,992 and 6,656 entities, 51 / 69, 67 / 77 and 82 / 78 ms: the line lies near 5,300 entities, four and a
-    // half times the warps co-resident at one host per warp)
-    const long long resident = (long long)c->dev_sms * std::max(1, tb::slot_kernel_blocks_per_sm(SW_STAGE, 1)) * TB_WARPS_PER_BLOCK * 9 / 4;
+    const long long resident = (long long)c->dev_sms * std::max(1, tb::slot_kernel_blocks_per_sm(SW_STAGE, 1)) * TB_WARPS_PER_BLOCK;
     tu.init(autotune, lanes, stage, entities, kmax, resident, [c](int l, int st) { return grid_for(c, l, st) > 0; });
 }
 

@@ -98,9 +98,11 @@ void world_units(Alive alive, const std::vector<std::array<int, 4>> &worlds, int
 
 // Launch-shape autotuning, for tb_run and the server. A shape is the hosts per warp and the frames a
 // warp stages per slot; no shape changes a result. It starts from one host per warp while the
-// entities fit the resident warps about twice (latency-bound: each host's serial
+// entities are at most four and a half times the resident warps (latency-bound: each host's serial
 // events are the slot's critical path), else 32 hosts per warp (throughput-bound: the lanes' memory
-// accesses overlap). Every `period` launches each shape still in the running
+// accesses overlap). Measured on 148 SMs (1,184 resident warps: the line at 5,328 entities), one / 32 hosts
+// per warp: 12 leaf-spine worlds, 2,940 entities, 178 / 417 ms; 16, 24 and 32 worlds of k=8, 3,328, 4,992 and
+// 6,656 entities, 51 / 69, 67 / 77 and 82 / 78 ms. Every `period` launches each shape still in the running
 // runs a probe of `probe` slots, and one whose device time per slot beats the current one's by
 // more than 5% takes over; a shape that loses a probe by more than 30% twice, or by more than 60%
 // once, is not probed again until every fourth round of probes, which probes all shapes (the load changes along a run).
@@ -144,7 +146,7 @@ struct ShapeTuner
                     shapes.push_back({x[0], x[1], 0, 0});
             // (one host per warp: with big switches (16 ports or more) the largest staging, else the one
             // that leaves more to L1. 32 hosts per warp: the smallest)
-            const int lanes0 = entities <= 2 * resident ? 1 : 32;
+            const int lanes0 = 2 * entities <= 9 * resident ? 1 : 32;
             const int stage0 = lanes0 == 1 ? (kmax >= 16 ? STAGE_BIG : STAGE_TWO) : STAGE_SMALL;
             for (size_t k = 0; k < shapes.size(); k++)
                 if (shapes[k].lanes == lanes0 && shapes[k].stage == stage0)
