@@ -2,14 +2,15 @@
 //
 // One cooperative launch runs up to `max_slots_per_launch` slots of every world in the batch.
 // Warps own entities for the whole launch (host units of `host_lanes` hosts, one thread each;
-// one switch per warp, one lane per port), so each entity's records stay in its SM's L1; link
-// messages cross SMs through L2 (ld/st.cg). A warp stages the link messages its unit reads in
-// shared memory first. Slots are separated by a grid barrier whose last arriving block does the
+// one switch per warp), so that an entity's records are its SM's alone; link messages cross SMs
+// through L2 (ld/st.cg). A warp stages the link messages its unit reads in
+// shared memory first. Slots are separated by a grid barrier (tb_sync.cuh) whose last arriving block does the
 // slot bookkeeping of the reference's ticket block (src/kernel.cuh:79-112): finish when every
 // message is done, else the exact idle skip to the earliest host wake-up when nothing was sent in
 // this or the previous slot. Every wait is bounded; a barrier that times out sets an error flag
 // and ends the launch.
 #include "tb_switch.cuh"
+#include "tb_sync.cuh"
 #include "tb_kernel.h"
 
 #include <algorithm>
@@ -34,27 +35,6 @@ __device__ __forceinline__ unsigned long long globaltimer()
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
-}
-
-// The barriers' words. Cross-SM data (link messages, the controller) is read from L2 (ld.cg,
-// volatile, atomics) and every entity's private state stays on its SM, so a wait needs no acquire,
-// and an arrival only a release: a full fence (__threadfence) on either side would also invalidate
-// the SM's L1, which holds the entities' records, for every warp of the SM in every slot.
-__device__ __forceinline__ unsigned add_release(unsigned *p, unsigned v)
-{
-    unsigned o;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
-    return o;
-}
-__device__ __forceinline__ void st_release(int64_t *p, int64_t v)
-{
-    asm volatile("st.release.gpu.global.s64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned ld_gen(const unsigned *p)
-{
-    unsigned v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
 }
 
 // An L1 line brought in ahead by a load whose value nobody waits for (prefetch.global.L1 left the
@@ -695,8 +675,10 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
             blk_next = ~0ull;
             blk_alive = 0;
             // grid barrier: the last block to arrive ends the slot and releases the others
-            g = ld_gen(&ctl->gen);
+            g = ld_relaxed(&ctl->gen);
             blk_last = add_release(&ctl->arrive, 1u) + 1 == gridDim.x;
+            if (blk_last)
+                acquire(&ctl->arrive);
         }
         __syncthreads();
         if (blk_last)
@@ -755,7 +737,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
         else if (threadIdx.x == 0)
         {
             long long spins = 0;
-            while (ld_gen(&ctl->gen) == g)
+            while (ld_relaxed(&ctl->gen) == g)
             {
                 if (++spins > BARRIER_SPIN_LIMIT)
                 {
@@ -766,6 +748,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) slot_kernel(
                 }
                 __nanosleep(64);
             }
+            acquire(&ctl->gen);
         }
         __syncthreads();
     }
@@ -849,7 +832,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
             int64_t t = 0, done = 0;
             if (lane == 0)
             {
-                t = __ldcg(&s.wctl[w].run);
+                t = ld_relaxed(&s.wctl[w].run);
                 done = s.unit_done[i];
             }
             t = __shfl_sync(FULL, t, 0);
@@ -860,6 +843,9 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
             if (done == t)
                 continue; // (done; its world's other units are not)
             ran = true;
+            if (lane == 0)
+                acquire(&s.wctl[w].run);
+            __syncwarp();
             unsigned ties = 0;
             if (host)
             {
@@ -874,7 +860,10 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
             {
                 s.unit_done[i] = t;
                 if (add_release(&s.wctl[w].arrive, 1u) + 1 == __ldcg(&s.wctl[w].units))
+                {
+                    acquire(&s.wctl[w].arrive);
                     world_close(s, w, t);
+                }
             }
             __syncwarp();
         }
@@ -885,7 +874,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, MIN_BLOCKS) free_kernel(
             idle = 0;
             continue;
         }
-        if (++idle > BARRIER_SPIN_LIMIT || __ldcg(&s.ctl->error))
+        if (++idle > BARRIER_SPIN_LIMIT || ld_relaxed((const unsigned *)&s.ctl->error))
         {
             if (lane == 0 && idle > BARRIER_SPIN_LIMIT)
             {
@@ -940,7 +929,7 @@ static bool smem_attr(int k)
 
 // The preferred shared-memory carveout, in percent of the SM's maximum: the shared memory of the
 // blocks a launch puts on one SM and no more, so that the rest of the SM's unified L1 / shared
-// memory is L1, where the units' records, ring heads and prefetched lines stay between slots.
+// memory is L1, which holds the units' records, ring heads and prefetched lines through a slot.
 static int carveout[K_N] = {-1, -1, -1, -1}; // the last ones set (-1: none)
 static void set_carveout(int k, int pct)
 {

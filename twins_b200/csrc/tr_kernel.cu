@@ -1,27 +1,21 @@
 // twins-b200: the RDMA model's slot kernel. One persistent cooperative launch runs many slots: a
-// warp owns NIC hosts and switches (the same ones every slot, so their records stay in its SM's L1)
+// warp owns NIC hosts and switches (the same ones every slot, so that their records are its SM's alone)
 // and runs each one's events of the slot (tr_sim.cuh: host_slot, switch_slot); a grid barrier ends
 // the slot and its last block applies the slot's end (finish, exact idle skip). Every wait is
 // bounded: a barrier that waits too long sets the run's error flag and the launch returns.
 // (reference: rdma_slot / rdma_persist / slot_end, src/rdma/rstep.cuh:3451-3577, 4020-4214)
 #include "tr_kernel.h"
 #include "tb_host.h"
+#include "tb_sync.cuh"
 
 namespace tr
 {
 
 constexpr long long BARRIER_SPIN_LIMIT = 1ll << 22; // polls of ~64 ns: a quarter of a second or more
 
-// What crosses SMs (frames, bucket tags, tail nodes, the controller) is read from L2, and an entity's
-// own records stay on its SM: the barrier releases what its block wrote, and needs no full fence
-// (__threadfence), which would invalidate the L1 that holds the records in every slot.
-__device__ __forceinline__ unsigned add_release(unsigned *p, unsigned v)
-{
-    unsigned o;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
-    return o;
-}
-__device__ __forceinline__ unsigned ld_volatile(const unsigned *p) { return *(const volatile unsigned *)p; }
+using tb::acquire;
+using tb::add_release;
+using tb::ld_relaxed;
 #ifdef TR_PROFILE
 __device__ __forceinline__ unsigned long long gtimer()
 {
@@ -113,8 +107,10 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32, MIN_BLOCKS) rdma_slot_kernel(
         unsigned g = 0;
         if (threadIdx.x == 0)
         {
-            g = ld_volatile(&ctl->gen);
+            g = ld_relaxed(&ctl->gen);
             blk_last = add_release(&ctl->arrive, 1u) + 1 == gridDim.x;
+            if (blk_last)
+                acquire(&ctl->arrive);
         }
         __syncthreads();
         if (threadIdx.x == 0)
@@ -140,7 +136,7 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32, MIN_BLOCKS) rdma_slot_kernel(
             else
             {
                 long long spins = 0;
-                while (ld_volatile(&ctl->gen) == g)
+                while (ld_relaxed(&ctl->gen) == g)
                 {
                     if (++spins > BARRIER_SPIN_LIMIT)
                     {
@@ -151,6 +147,7 @@ __global__ void __launch_bounds__(RDMA_WARPS * 32, MIN_BLOCKS) rdma_slot_kernel(
                     }
                     __nanosleep(64);
                 }
+                acquire(&ctl->gen);
             }
         }
         __syncthreads();

@@ -2129,8 +2129,7 @@ TR_HD bool switch_slot(const RSim &s, int x, int64_t t, const SwWork &w, int lan
 // After every entity ran slot t: the run ends when every flow is done or at the stop time; a slot
 // in which nothing was sent or held goes on at the earliest host event or frame arrival; nothing
 // left at all ends the run (quiescence). (reference: slot_end, src/rdma/rstep.cuh:3451-3577)
-// (activity, next_wake and flows_done: the entities' sums of the slot, read by the caller; the
-// controller is another SM's in the next slot: no L1 copy of it is read)
+// (activity, next_wake and flows_done: the entities' sums of the slot, read by the caller)
 TR_HD void slot_close(const RSim &s, int64_t t, unsigned activity, unsigned long long next_wake, unsigned flows_done)
 {
     volatile RCtl &c = *s.ctl;
