@@ -84,3 +84,33 @@ def test_rdma_kept_batches_of_different_switches(native_lib):
         _, fct = sim.rdma_results(0)
         assert (fct == want(name, len(fct))).all(), name
         sim.close()
+
+
+def test_rdma_repeated_runs_identical(native_lib):
+    """A batch's runs fill the device arrays of the run before again: a second run, one that max_slots cuts
+    short, and one after it give what a fresh batch gives, results and all counters."""
+    names = ["ft8_incast32_dcqcn_pfc", "ft4_uniform80_hpcc"]
+
+    def got(sim):
+        return [sim.rdma_results(w)[1] for w in range(len(names))], sim.rdma_counters()
+
+    def batch():
+        sim = api.Simulator()
+        for name in names:
+            sim.add_rdma_world(*inputs(name))
+        return sim
+
+    with batch() as sim:
+        assert sim.run() == api.TB_OK
+        fresh = got(sim)
+        for name, fct in zip(names, fresh[0]):
+            assert (fct == want(name, len(fct))).all(), name
+    with batch() as sim:
+        sim.run(max_slots=40)
+        cut = got(sim)
+        assert any((fct < 0).any() for fct in cut[0])
+    with batch() as sim:
+        for max_slots, expected in ((0, fresh), (40, cut), (0, fresh), (0, fresh)):
+            sim.run(max_slots)
+            fct, counters = got(sim)
+            assert all((a == b).all() for a, b in zip(fct, expected[0])) and counters == expected[1]

@@ -4,6 +4,7 @@
 // until every flow is done, the stop time or quiescence, and read back.
 // (reference: the driver of src/rdma/rmain.cu:1023-2373)
 #include "tr_capi.h"
+#include "tr_arrays.h"
 #include "tr_kernel.h"
 #include "tr_layout.h"
 
@@ -16,65 +17,15 @@ namespace tr
 
 namespace
 {
-// The run's arrays that start as set-up images, the ones that start zeroed, and the tail ring. A run
-// takes them in one order and of one size (but for a tail ring that grew), so the next run of the
-// batch fills the same memory again: allocating and freeing some forty arrays, gigabytes in all, took
-// 10 ms of a small run and up to 100 ms when the driver was slow about it.
-struct DevArrays
+struct DeviceMem
 {
-    struct Piece
-    {
-        void *p;
-        size_t bytes;
-    };
-    std::vector<Piece> mem;
-    size_t at = 0, bytes = 0; // the next piece; the bytes taken by this run
-    cudaStream_t stream = nullptr;
-    ~DevArrays() { release(); }
-    void release()
-    {
-        for (Piece &m : mem)
-            cudaFree(m.p);
-        mem.clear();
-        at = bytes = 0;
-    }
-    void begin(cudaStream_t s)
-    {
-        stream = s;
-        at = bytes = 0;
-    }
-    template <class T>
-    bool take(T **p, size_t n)
-    {
-        const size_t b = sizeof(T) * (n ? n : 1);
-        if (at == mem.size())
-            mem.push_back({nullptr, 0});
-        Piece &m = mem[at++];
-        if (m.bytes != b)
-        {
-            cudaFree(m.p);
-            m = {nullptr, 0};
-            if (cudaMalloc(&m.p, b) != cudaSuccess)
-                return false;
-            m.bytes = b;
-        }
-        *p = (T *)m.p;
-        bytes += b;
-        return true;
-    }
-    template <class T>
-    bool zeroed(T **p, size_t n)
-    {
-        return take(p, n) && cudaMemsetAsync(*p, 0, sizeof(T) * (n ? n : 1), stream) == cudaSuccess;
-    }
-    template <class T>
-    bool copy(T **p, const std::vector<T> &v)
-    {
-        if (v.empty())
-            return zeroed(p, 0);
-        return take(p, v.size()) && cudaMemcpyAsync(*p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream) == cudaSuccess;
-    }
+    using Stream = cudaStream_t;
+    static bool alloc(void **p, size_t n) { return cudaMalloc(p, n) == cudaSuccess; }
+    static void release(void *p) { cudaFree(p); }
+    static bool zero(void *p, size_t n, Stream s) { return cudaMemsetAsync(p, 0, n, s) == cudaSuccess; }
+    static bool copy(void *p, const void *from, size_t n, Stream s) { return cudaMemcpyAsync(p, from, n, cudaMemcpyHostToDevice, s) == cudaSuccess; }
 };
+using DevArrays = RunArrays<DeviceMem>;
 } // namespace
 
 struct RdmaRun
