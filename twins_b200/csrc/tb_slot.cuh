@@ -1,9 +1,9 @@
-// twins-b200: one slot of a host and of a switch.
+// twins-b200: one slot of a host, and a switch's routes.
 //   host_step   (reference: src/step.cuh:2250-2528) one thread per host: every event of the host
 //               in [t us, t+1 us) in ns-3's order: arrivals, timers, application starts
-//   switch_step (reference: src/step.cuh:2530-2886) one warp per switch, one lane per port:
-//               ingress windows -> routes (per-flow ECMP or MRG32k3a spraying) -> counting sort to
-//               egress ports -> per-egress ordering by (time, ns-3 order) -> RED enqueue -> starts
+//   route, ...  (reference: src/step.cuh:2530-2705) a frame's egress port (per-flow ECMP or a spraying
+//               choice, link failures) and ns-3's order of simultaneous arrivals; the switch's slot itself
+//               is tb_switch.cuh's and tb_kernel.cu's switch_step
 #pragma once
 #include "tb_tcp.cuh"
 

@@ -251,6 +251,10 @@ __device__ __forceinline__ unsigned long long prof_now()
 #define TB_PHASE(i)
 #endif
 
+// Of these arrays msg, msg_tag, ctl and wctl are written by one SM and read by others in the next slots: their
+// readers go to L2 (ld.cg, volatile, atomics), after the barrier's acquire (tb_sync.cuh). Every other array's
+// entries are one entity's, which one warp owns for the launch, or constant (a sender record's hashes, which
+// switches of a topology file read, never change). ev and ev_w are only added to.
 struct Sim
 {
     int W, H, S, P, L, C, M;

@@ -246,7 +246,10 @@ enum
     EV_N = 40
 };
 
-// every array of a run (device pointers in the kernel, host pointers in the CPU harness)
+// Every array of a run (device pointers in the kernel, host pointers in the CPU harness). Written by one SM and
+// read by others in later slots: msg, msg_cnt, pend, tail and ctl (through L2, after the barrier's acquire,
+// tb_sync.cuh); ev and the counters of tail and tx are only added to. The other entries are one entity's, or
+// constant.
 struct RSim
 {
     int H, S, F, W, P; // hosts, switches, flows, worlds, switch ports
