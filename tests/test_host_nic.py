@@ -1,9 +1,13 @@
-"""A host's sending end on the CPU: tests/host_nic.cpp, built with g++ over twins_b200/csrc/tb_tcp.cuh and
-tb_egress.cuh in the enqueue trace's build. The list that a host with a warp of its own plays through its
-NIC (HostNic) against the device frame by frame (Egress): frames sent and held, counters, and the traced
-enqueues' endpoints, which a frame offered by a ScheduleNow'd event of its instant had swapped."""
+"""The sending ends on the CPU, built with g++ over the library's headers in the enqueue trace's build: each
+form that takes a slot at a time against the device frame by frame (Egress). tests/host_nic.cpp: the list
+that a host with a warp of its own plays through its NIC (HostNic), whose traced enqueues had source and
+destination swapped for a frame offered by a ScheduleNow'd event of its instant. tests/switch_port.cpp: a
+switch port's slot staged in shared memory (sw_egress_staged)."""
+import pytest
+
 from test_sent_list import run_check
 
 
-def test_host_nic_equals_egress(tmp_path):
-    run_check(tmp_path, "host_nic")
+@pytest.mark.parametrize("form", ["host_nic", "switch_port"])
+def test_sending_end_equals_egress(tmp_path, form):
+    run_check(tmp_path, form)
