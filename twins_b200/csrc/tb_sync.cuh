@@ -10,7 +10,7 @@
 // A wait polls with relaxed loads and acquires once, when it is over: an acquire empties the SM's L1,
 // which holds the records of the entities of all its warps, and an entity's first events of the slot
 // then read them from L2. Measured, against waits without an acquire (the same results on every world
-// tried, but PTX then orders none of what is read after the wait): 3-8% of a TCP run (k=8 NewReno 69.6 /
+// tried, but PTX then orders none of what is read after the wait): 3-10% of a TCP run (k=8 NewReno 69.6 /
 // 75.7 ms, 96 k=8 worlds 99.2 / 106 ms, k=16 68.6 / 70.5 ms), 0-2% of an RDMA run. A fence at the arrival that
 // closes the slot instead of the acquiring load costs up to 3% more, acquiring polls up to 10% more (k=16
 // 77.9 ms), and bringing the records back by loads ahead of the events gains nothing.
