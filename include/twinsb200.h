@@ -174,7 +174,8 @@ int tb_results(tb_ctx *ctx, int world, long long *established_ns, long long *com
 /* Counters of a world (n <= 16): drops, marks, retransmissions, RTOs, undecided ties, host
  * packet-events, switch packet-events, overflow counts (active lists, timers, rings,
  * out-of-order blocks, tx-cap), barrier timeouts, sender-side host packet-events, frames hosts
- * emitted (reference counters, src/main.cu:1064-1075). */
+ * emitted (reference counters, src/main.cu:1064-1075); the trace build alone also counts the switch slots
+ * of more frames than the staging area holds. */
 int tb_counters(tb_ctx *ctx, int world, unsigned long long *out, int n);
 
 /* Per flow row of a world: the ECMP hashes in use (reference --hash_check, src/main.cu:755-768). */
